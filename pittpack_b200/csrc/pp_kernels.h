@@ -53,6 +53,8 @@ struct PPLinePassArgs {
     const void* cs2;   // family twiddles in the kernel's precision
     int in_cplx, out_cplx;
     int vec16;          // power-of-two kernel: src and its run starts are 16-byte aligned
+                        // (half-length kernel: aligned to its widest load)
+    int vec_out;        // half-length kernel: dst and its runs are aligned to its widest store
     int half;           // power-of-two periodic x pass of a real RHS on half spectra
                         // (N/2 + 1 complex per line): forward real -> half, inverse half -> real
     // refinement epilogue of the inverse x pass (acc != null): the real part v
@@ -113,6 +115,15 @@ cudaError_t pp_launch_line_pass_pow2(const PPLinePassArgs& a, bool inverse, bool
 // 9 2^k (144 .. 1152) and 15 2^k (240 .. 960):
 // complex FFT lines per CTA (0 = not covered), and the FP64 / FP32 launches
 int pp_lpm_lpc(int n);
+// the real families and the periodic half spectra through a complex FFT of
+// half the length (pp_rhalf.cuh): data lines per CTA tile (0 = not covered),
+// whether a pass takes that kernel, and the pass (a.tw and a.cs2 in its
+// precision, strides and output strides set; out strides of 0: the input's)
+int pp_rh_lines(int n, bool strided);
+bool pp_rh_covers(const PPLinePassArgs& a, bool inverse, bool strided, bool out_cplx);
+cudaError_t pp_rh_line_pass(PPLinePassArgs a, bool inverse, bool strided, bool in_cplx, bool out_cplx, bool fp32,
+                            cudaStream_t st);
+cudaError_t pp_launch_line_pass_rh_f32(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st);
 cudaError_t pp_launch_line_pass_mixed(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st);
 cudaError_t pp_launch_line_pass_mixed_f32(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st);
 // 9 2^k and 15 2^k (144 .. 1152), called by the two above

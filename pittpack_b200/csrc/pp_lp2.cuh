@@ -1,5 +1,6 @@
 // Transform pass for line lengths N = m 2^k (m = 1, 3, 5, 9, 15; the FFT's
-// power-of-two factor at least 8): the same four passes and the same
+// power-of-two factor at least 8; the real families and half spectra of
+// N = 32 .. 1024, m = 1, take pp_rhalf.cuh): the same four passes and the same
 // per-family pre/post-processing as pp_linepass.cu (see the reference
 // citations there), built on the register-resident FFT of pp_fftreg.cuh and
 // specialised at compile time on the length and the boundary family, so that
@@ -713,10 +714,8 @@ __global__ void __launch_bounds__(LPC * N / 8, lpm_min_blocks(LPC * N / 8)) lpm_
 {
     lp2_body<Real, N, LPC, FAM, INVERSE, STRIDED>(a);
 }
-// the periodic family's 512-point FP64 instances (complex lines, half
-// spectra): bounded to 48 registers, five CTAs of 256 threads per SM
-// (measured faster; the real families' instances spill under the same bound
-// and are not)
+// the periodic family's 512-point FP64 instance (complex lines): bounded to 48
+// registers, five CTAs of 256 threads per SM (measured faster)
 template <typename Real, int N, int LPC, int FAM, bool INVERSE, bool STRIDED>
 __global__ void __launch_bounds__(LPC * N / 8, 5) lp2b_kernel(PPLinePassArgs a)
 {
@@ -725,7 +724,7 @@ __global__ void __launch_bounds__(LPC * N / 8, 5) lp2b_kernel(PPLinePassArgs a)
 template <typename Real, int N, int LPC, int FAM, bool INVERSE, bool STRIDED>
 constexpr auto pass_kernel()
 {
-    if constexpr (N == 512 && (FAM == F_FFT || FAM == F_R2C || FAM == F_C2R) && std::is_same<Real, double>::value)
+    if constexpr (N == 512 && FAM == F_FFT && std::is_same<Real, double>::value)
         return lp2b_kernel<Real, N, LPC, FAM, INVERSE, STRIDED>;
     else if constexpr ((N & (N - 1)) == 0) return lp2_kernel<Real, N, LPC, FAM, INVERSE, STRIDED>;
     else return lpm_kernel<Real, N, LPC, FAM, INVERSE, STRIDED>;
@@ -766,6 +765,11 @@ cudaError_t launch_half(const PPLinePassArgs& a, cudaStream_t st)
 template <typename Real, int N, int LPC>
 cudaError_t launch_n(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st)
 {
+    if constexpr (N >= 32 && N <= 1024 && (N & (N - 1)) == 0) {
+        // the real families and the half spectra of these lengths: pp_rhalf.cuh
+        return a.kind == PP_KIND_FFT && !a.half ? launch_fam<Real, N, LPC, F_FFT>(a, inverse, strided, st)
+                                                : cudaErrorInvalidValue;
+    } else {
     if (a.half && a.kind == PP_KIND_FFT) {
         if (strided) return cudaErrorInvalidValue;
         return inverse ? launch_half<Real, N, LPC, F_C2R>(a, st) : launch_half<Real, N, LPC, F_R2C>(a, st);
@@ -775,6 +779,7 @@ cudaError_t launch_n(const PPLinePassArgs& a, bool inverse, bool strided, cudaSt
     case PP_KIND_DCT2: return launch_fam<Real, N, LPC, F_DCT2>(a, inverse, strided, st);
     case PP_KIND_FFT: return launch_fam<Real, N, LPC, F_FFT>(a, inverse, strided, st);
     default: return launch_fam<Real, N, LPC, F_Q4>(a, inverse, strided, st);
+    }
     }
 }
 

@@ -207,6 +207,11 @@ cudaError_t na_line_pass(PPLinePassArgs a, const NaDir& d, const double2* tw, co
     a.fft = d.fft;
     a.fft.tw = tw;
     a.cs = cs;
+    if (pp_rh_covers(a, inverse, strided, out_cplx)) {
+        a.tw = tw;
+        a.cs2 = cs;
+        return pp_rh_line_pass(a, inverse, strided, in_cplx, out_cplx, false, st);
+    }
     const int lpc2 = pp_lp2_lpc(d.n), lpc = lpc2 ? lpc2 : pp_lpm_lpc(d.n);
     if (lpc > 0) {
         a.tw = tw;

@@ -588,6 +588,11 @@ cudaError_t line_pass(PPLinePassArgs a, const DirTables& d, bool inverse, bool s
         a.tiles_per_plane = (a.nlines + a.L - 1) / a.L;
         return pp_launch_line_pass(a, inverse, strided, in_cplx, out_cplx, st, true);
     }
+    if (pp_rh_covers(a, inverse, strided, out_cplx)) {
+        a.tw = fp32 ? d.twf.p : d.tw.p;
+        a.cs2 = fp32 ? d.csf.p : d.cs.p;
+        return pp_rh_line_pass(a, inverse, strided, in_cplx, out_cplx, fp32, st);
+    }
     if (lpc > 0) {
         // data lines per tile: one per complex FFT line for the full complex
         // family, two (packed real lines) for the others and the half spectra
@@ -666,12 +671,16 @@ int reg_lines(int n)
     const int lpc = pp_lp2_lpc(n);
     return lpc ? lpc : pp_lpm_lpc(n);
 }
+// data lines per tile of the y pass (0: the generic kernel)
+int y_tile_lines(int n, bool cplx)
+{
+    if (!cplx && pp_rh_lines(n, true)) return pp_rh_lines(n, true);
+    return cplx ? reg_lines(n) : 2 * reg_lines(n);
+}
 int z_tile_width(const pp_solver_s* h, bool s_cplx, int ncol)
 {
     if (h->opt.z_solver != PP_ZSOLVE_DIRECT || h->slab) return 0;
-    const int lpc = reg_lines(h->ny);
-    if (lpc == 0) return 0;
-    const int dl = s_cplx ? lpc : 2 * lpc;
+    const int dl = y_tile_lines(h->ny, s_cplx);
     if (dl < 2 || dl > 16 || ncol % dl != 0) return 0;
     if (h->tune.zsolve_tile != 0 && h->tune.zsolve_tile != dl) return 0;
     int ts = 0, threads = 0;
@@ -688,8 +697,8 @@ int z_tile_width(const pp_solver_s* h, bool s_cplx, int ncol)
 int half_spectrum_cols(const pp_solver_s* h)
 {
     if (h->tx.kind != PP_KIND_FFT || h->rhs_complex || h->nx < 32 || reg_lines(h->nx) == 0) return 0;
-    const int lpy = reg_lines(h->ny);
-    int q = lpy ? (h->ty.kind == PP_KIND_FFT ? lpy : 2 * lpy) : 1;
+    int q = y_tile_lines(h->ny, h->ty.kind == PP_KIND_FFT);
+    if (q == 0) q = 1;
     if (q > 16) q = 16;
     const int c = ((h->nx / 2 + 1 + q - 1) / q) * q;
     return c <= h->nx ? c : 0;
