@@ -155,12 +155,9 @@ struct PPZArgs {
     int* err;           // counts CTAs whose bounded waits ran out (may be null)
 };
 
-// lanes that share one z system (a power of two <= 32)
-int pp_zsolve_lanes(int nz, bool cplx, bool large = false);
-// grids of at least this many z systems (kx x ky columns) keep uneven row
-// counts in registers too (the register capacity path of the z solve)
-#define PP_Z_LARGE_SYSTEMS 65536L
-bool pp_zsolve_large(long systems);
+// lanes that share one z system (a power of two <= 32) of a grid with that
+// many systems
+int pp_zsolve_lanes(int nz, bool cplx, long systems);
 // systems per CTA and threads per CTA of the z solve
 void pp_zsolve_config(int nz, bool cplx, int nx, int* TS, int* threads);
 // the same for a chosen lane count (0 or invalid: the default); the launch

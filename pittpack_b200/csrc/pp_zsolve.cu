@@ -35,11 +35,15 @@
 //     in the lanes' last unknowns, solved by parallel cyclic reduction over
 //     warp shuffles (periodic systems through Sherman-Morrison); each lane
 //     then recovers its interior rows;
-//   * where every lane keeps exactly 10, 12, 16, 20, 24 or 32 rows in registers, they form two
-//     blocks of half that length whose sweeps run side by side (two
-//     independent FP64 recurrences per lane: the sweeps are bound by the
-//     latency of their dependent operations), and one more elimination step
-//     on the lane reduces the two blocks' rows to one before the shuffles.
+//   * where a lane keeps 9 .. 34 rows (complex 9 .. 19) in registers, they form
+//     two blocks whose sweeps run side by side (two independent FP64
+//     recurrences per lane: the sweeps are bound by the latency of their
+//     dependent operations), and one more elimination step on the lane reduces
+//     the two blocks' rows to one before the shuffles.  Row counts that do not
+//     divide by the lanes, or are odd, shorten the second block by one or two
+//     rows (before, they kept one block of up to 32 rows on grids of 256^2
+//     systems and their rows in shared memory on smaller ones: 192^3 z solve
+//     0.064 -> 0.028 ms, 200^3 0.089 -> 0.056, 96^3 0.019 -> 0.011).
 #include <type_traits>
 
 #include "pp_common.cuh"
@@ -239,13 +243,16 @@ PP_D T zsolve_reduced(double ra, double rb, double rc, T rd, int lane, int P, bo
 // a block of H rows (gamma_i, alpha_i, i < H); d0 is row 0's right-hand side
 // (after the periodic zero-mode averaging); row 0 of the system is the first
 // row of A on lane 0 and row nz - 1 the last row of B on lane P - 1.
-template <int MT, typename T>
-PP_D void zsolve_split(T (&xr)[MT], const double2* tab, T d0, bool live, bool clear, int lane, int P,
+// UNEV: a lane has M = MT, MT - 1 or MT - 2 rows; block B is the shorter one
+// (HB = M - H rows), the branches on it are confined to its last three rows.
+template <int MT, bool UNEV, typename T>
+PP_D void zsolve_split(T (&xr)[MT], const double2* tab, T d0, int M, bool live, bool clear, int lane, int P,
                        bool periodic, double lam, double A0, double B0, double C0, double AN, double BN,
                        double CN)
 {
     constexpr int H = MT / 2;
-    static_assert(H >= 4, "blocks of at least four rows");
+    static_assert(H >= (UNEV ? 5 : 4), "blocks of at least four rows, three in the shorter one");
+    const int HB = UNEV ? M - H : H;
     const double* tg = reinterpret_cast<const double*>(tab);  // gamma_i = tg[2i], alpha_i = tg[2i+1]
     const bool last = lane == P - 1;
     // ---- forward sweeps of A and B ----------------------------------------------------
@@ -257,8 +264,17 @@ PP_D void zsolve_split(T (&xr)[MT], const double2* tab, T d0, bool live, bool cl
         for (int i = 1; i < H; ++i) {
             const double ga = tg[2 * i];
             const T nA = (i == 1) ? zmul(ga, xr[i]) : zmul(ga, zsub(xr[i], dA));
-            T nB;
-            if (i == H - 1 && last) {
+            T nB = zzero<T>();
+            // (rows above H - 4 may be B's last one, or past it)
+            const bool ends = UNEV && i > H - 4 ? i == HB - 1 : i == H - 1;
+            const bool past = UNEV && i > H - 3 && i > HB - 1;
+            if (past) {
+                xr[i] = nA;
+                dA = nA;
+                gA = ga;
+                continue;
+            }
+            if (ends && last) {
                 // the system's last row closes B on the last lane
                 const double p = 1.0 / (BN - AN * gB);
                 aB = -AN * tg[2 * (i - 1) + 1] * p;
@@ -276,22 +292,29 @@ PP_D void zsolve_split(T (&xr)[MT], const double2* tab, T d0, bool live, bool cl
             gA = ga;
         }
         aA = tg[2 * (H - 1) + 1];
-        if (!lastB) aB = aA;
+        if (!lastB) aB = UNEV ? tg[2 * (HB - 1) + 1] : aA;
     }
     // ---- backward sweeps: row 1 of a block in terms of its first and last unknowns
-    double br = 0.0, cr = 0.0;
+    double br = 0.0, cr = 0.0, brB = 0.0, crB = 0.0;
     T rA = zzero<T>(), rB = zzero<T>();
     if (live) {
         const double2 t2 = tab[H - 2];
-        br = t2.x;
-        cr = t2.y;
+        br = brB = t2.x;
+        cr = crB = t2.y;
+        if (UNEV) {
+            const double2 u2 = tab[HB - 2];
+            brB = u2.x;
+            crB = u2.y;
+        }
         rA = xr[H - 2];
         rB = xr[MT - 2];
 #pragma unroll
         for (int i = H - 3; i >= 1; --i) {
             const double g = tg[2 * i];
             rA = zsub(xr[i], zmul(g, rA));
-            rB = zsub(xr[H + i], zmul(g, rB));
+            // (UNEV: B's sweep starts at its row HB - 2)
+            if (UNEV && i > H - 5 && i >= HB - 2) rB = xr[H + i];
+            else rB = zsub(xr[H + i], zmul(g, rB));
         }
     }
     // ---- E0 of both blocks (A's first row is the system's row 0 on lane 0) -----------
@@ -300,8 +323,8 @@ PP_D void zsolve_split(T (&xr)[MT], const double2* tab, T d0, bool live, bool cl
     const double qA = 1.0 / (b0 - c0 * br);
     const double e0aA = a0 * qA, e0cA = -c0 * cr * qA;
     const T e0dA = zmul(qA, zsub(d0, zmul(c0, rA)));
-    const double qB = 1.0 / (lam - br);
-    const double e0aB = qB, e0cB = -cr * qB;
+    const double qB = 1.0 / (lam - brB);
+    const double e0aB = qB, e0cB = -crB * qB;
     const T e0dB = zmul(qB, zsub(live ? xr[H] : zzero<T>(), rB));
     // ---- rows of the blocks' last unknowns --------------------------------------------
     // l_A:  raA l_B(prev lane) + rbA l_A + rcA l_B = rdA
@@ -334,13 +357,20 @@ PP_D void zsolve_split(T (&xr)[MT], const double2* tab, T d0, bool live, bool cl
     }
     T xa = lA, xb = lB;
     xr[H - 1] = lA;
-    xr[MT - 1] = lB;
+    if (UNEV) {
+#pragma unroll
+        for (int i = H - 3; i < H; ++i)
+            if (i == HB - 1) xr[H + i] = lB;
+    } else {
+        xr[MT - 1] = lB;
+    }
 #pragma unroll
     for (int i = H - 2; i >= 1; --i) {
         const double2 ti = tab[i];
         xa = zsub(zsub(xr[i], zmul(ti.y, fA)), zmul(ti.x, xa));
-        xb = zsub(zsub(xr[H + i], zmul(ti.y, fB)), zmul(ti.x, xb));
         xr[i] = xa;
+        if (UNEV && i > H - 4 && i > HB - 2) continue;
+        xb = zsub(zsub(xr[H + i], zmul(ti.y, fB)), zmul(ti.x, xb));
         xr[H + i] = xb;
     }
     xr[0] = fA;
@@ -368,6 +398,9 @@ PP_HD ZLayout zlayout(int TS, int nz, int P, bool cplx, int nthreads, bool g32 =
     L.groups = nthreads / P;
     L.tile_off = 0;
     L.tab_off = (size_t)TS * L.pitch * e;
+    // (the bulk-copied tile: a chunk of the lane's rows and 16 bytes per lane)
+    const size_t chunks = (size_t)P * (((size_t)(nz + P - 1) / P) * TS * e + 16);
+    if (chunks > L.tab_off) L.tab_off = chunks;
     L.tab_off = (L.tab_off + 15) & ~(size_t)15;
     // scratch of the pivot-table build: the b_i recurrence of every system
     L.red_off = L.tab_off + (size_t)TS * L.mmax * 16;
@@ -408,11 +441,10 @@ PP_D TG zdown(T v)
 // all arithmetic stays FP64 (the shared tile too, except in the bulk-copied
 // chunks, which hold the stored elements).  MT > 0: every lane keeps its rows
 // in registers through the three sweeps, reading and writing its rows of the
-// tile once -- exactly MT rows each (CAP = false, nz = P MT, MT = 8, 10, 12, 16, 20, 24, 32),
-// or at most MT (CAP = true, MT = 8, 12, 16, 24, 32: M = nz / P or one more,
-// the registers indexed statically under i < M guards); MT = 0: any nz, the
-// sweeps work on the tile in shared memory.  SPLIT: exactly MT = 10, 12, 16, 20, 24 or 32
-// rows per lane, swept as two half blocks (zsolve_split).
+// tile once -- exactly MT rows each (CAP = false, nz = P MT), or M = nz / P or
+// one more under static i < M guards (CAP = true: at most 8 in one block, MT - 2
+// to MT in the split solve); MT = 0: any nz, the sweeps work on the tile in
+// shared memory.  SPLIT: two half blocks (zsolve_split).
 template <bool CPLX, bool G32, int MT, bool CAP, bool SPLIT>
 PP_D void zsolve_body(PPZArgs a)
 {
@@ -436,10 +468,8 @@ PP_D void zsolve_body(PPZArgs a)
     // or the z-tiled one, where this CTA's tile is one contiguous block
     const long plane = a.tiled ? (long)a.TS : (long)nx * ny;
     const long col0 = a.tiled ? (long)blockIdx.x * nz * a.TS : (long)ky * nx + kx0;
-    // Bulk-copied tiles: z-tiled, rows in registers, and either the split
-    // kernels or complex spectra with uneven row counts (where complex uneven
-    // rows gained 0.30 -> 0.28 ms at 384^3, real ones lost 3 %).  Each lane
-    // block of the tile (the lane's rows x TS systems, contiguous in global
+    // Bulk-copied tiles: z-tiled, and the split kernels or complex spectra with
+    // uneven rows in registers.  Each lane block of the tile (the lane's rows x TS systems, contiguous in global
     // memory) moves as one bulk copy (the copy engine, not the LSU pipe) into a
     // chunk of shared memory,
     // the chunks 16 bytes past the longest block so that the lanes of a phase
@@ -449,7 +479,7 @@ PP_D void zsolve_body(PPZArgs a)
     // registers.  Lane L's block is rows L brows + min(L, brem) on, brows + 1
     // of them for the first brem lanes, brows for the rest.
     using TG = typename std::conditional<G32, T32, T>::type;  // element in global memory
-    const int brows = SPLIT ? MT : nz / P, brem = SPLIT ? 0 : nz - brows * P;  // split: nz = P MT
+    const int brows = SPLIT && !CAP ? MT : nz / P, brem = SPLIT && !CAP ? 0 : nz - brows * P;
     const int crow = a.TS * (int)sizeof(TG);                  // bytes of one tile row
     const int cpitch = (brows + (brem ? 1 : 0)) * crow + 16;
     const bool bulk = (SPLIT || (CAP && CPLX)) && a.tiled && ts == a.TS && crow % 16 == 0 &&
@@ -634,17 +664,16 @@ PP_D void zsolve_body(PPZArgs a)
         }
 
         if constexpr (SPLIT) {
-            static_assert(EXACT, "the split solve keeps exactly MT rows per lane");
             T d0 = zzero<T>();
             if (live) {
                 d0 = xr[0];
                 if (lane == 0 && periodic && pin) {
-                    const T last = bulk ? zup<T>(reinterpret_cast<const TG*>(zsm_raw + (size_t)(P - 1) * cpitch)[(MT - 1) * a.TS + s])
+                    const T last = bulk ? zup<T>(reinterpret_cast<const TG*>(zsm_raw + (size_t)(P - 1) * cpitch)[(brows - 1) * a.TS + s])
                                         : col[zpos(nz - 1)];
                     d0 = zmul(0.5, zadd(d0, last));
                 }
             }
-            zsolve_split<MT>(xr, tab, d0, live, zero && a.skip_zero, lane, P, periodic, lam, A0, B0, C0, AN, BN, CN);
+            zsolve_split<MT, CAP>(xr, tab, d0, M, live, zero && a.skip_zero, lane, P, periodic, lam, A0, B0, C0, AN, BN, CN);
         } else {
             // ---- forward sweep of the lane's block -------------------------------------
             // row i (i >= 1) becomes alpha_i x_0 + x_i + gamma_i x_{i+1} = delta_i; delta
@@ -861,45 +890,44 @@ __global__ void __launch_bounds__(PP_Z_THREADS) zsolve_kernel(PPZArgs a)
 // it gains (0.33 -> 0.36 ms).  A separate kernel: naming a minimum of one
 // CTA per SM in the other kernels' launch bounds lets the compiler spend
 // more registers on them than the one-argument form does.
-template <bool CPLX, bool G32, int MT>
+template <bool CPLX, bool G32, int MT, bool CAP>
 __global__ void __launch_bounds__(PP_Z_THREADS, 2) zsolve_split_r128_kernel(PPZArgs a)
 {
-    zsolve_body<CPLX, G32, MT, false, true>(a);
+    zsolve_body<CPLX, G32, MT, CAP, true>(a);
 }
 // the split kernel a launch takes (only that one is compiled)
-template <bool CPLX, bool G32, int MT>
+template <bool CPLX, bool G32, int MT, bool CAP>
 void (*split_kernel())(PPZArgs)
 {
-    if constexpr (CPLX || !G32) return zsolve_split_r128_kernel<CPLX, G32, MT>;
-    else return zsolve_kernel<CPLX, G32, MT, false, true>;
+    if constexpr (CPLX ? MT <= 16 : (!G32 && MT <= 32)) return zsolve_split_r128_kernel<CPLX, G32, MT, CAP>;
+    else return zsolve_kernel<CPLX, G32, MT, CAP, true>;
 }
 }  // namespace
 
-int pp_zsolve_lanes(int nz, bool cplx, bool large)
+int pp_zsolve_lanes(int nz, bool cplx, long systems)
 {
-    // about 32 rows per lane (16 for complex data, whose tile is twice as
-    // large, so that a CTA still keeps every group busy).  Grids with many
-    // systems (large) take the fewest lanes that leave at most that many rows,
-    // so that any nz keeps its rows in registers; smaller grids keep more
-    // resident CTAs with the shared-memory rows (batches of small grids run
-    // concurrently, where occupancy counts more)
-    const int rows = cplx ? 16 : 32;
+    // the fewest lanes that keep every lane's rows in registers: fewer lanes mean
+    // fewer steps of the reduced system's PCR per row (384 x 384 x 272, real: 8
+    // lanes of 34 rows 0.164 ms, 16 of 17 0.209; 192 x 160 x 144, complex: 8 of 18
+    // rows 0.041 ms, 16 of 9 0.052), up to the counts whose registers leave too
+    // few warps (384 x 384 x 288: 8 of 36 rows 0.246 ms, 16 of 18 0.211; 192 x
+    // 192 x 160, complex: 8 of 20 0.058 ms, 16 of 10 0.048)
+    const int rows = cplx ? 19 : 34;
     int P = 1;
-    if (large)
-        while (P < 32 && (nz + P - 1) / P > rows) P *= 2;
-    else
-        while (P < 32 && 2 * P <= nz / rows) P *= 2;
+    while (P < 32 && (nz + P - 1) / P > rows) P *= 2;
+    // few systems: more lanes with shorter sweeps, while the GPU has room for
+    // them and a lane keeps at least nine rows (64^3: 4 lanes of 16 rows take 2 us
+    // less than 2 of 32; 192 x 192 planes are past this)
+    while (P < 32 && systems * P < 32768 && nz / (2 * P) >= 9) P *= 2;
     while (P > 1 && P > nz / 2) P /= 2;
     return P;
 }
-
-bool pp_zsolve_large(long systems) { return systems >= PP_Z_LARGE_SYSTEMS; }
 
 // launch shape: systems per CTA (one lane group each) and threads per CTA,
 // keeping the CTA within ~56 KB of shared memory so about four fit on an SM
 void pp_zsolve_config(int nz, bool cplx, int nx, int* TS, int* threads)
 {
-    const int P = pp_zsolve_lanes(nz, cplx, false);
+    const int P = pp_zsolve_lanes(nz, cplx, 1);
     int ts = PP_Z_THREADS / P;
     auto bytes = [&](int t) {
         const int th = t * P < 32 ? 32 : t * P;
@@ -928,7 +956,7 @@ size_t pp_zsolve_smem_p(int TS, int nz, bool cplx, int P)
 // systems per CTA (0: as many as fit ~56 KB of shared memory)
 void pp_zsolve_config_p(int nz, bool cplx, int nx, int lanes, int* TS, int* threads, int systems, int ny)
 {
-    const int P = pp_zsolve_valid_lanes(nz, lanes) ? lanes : pp_zsolve_lanes(nz, cplx, pp_zsolve_large((long)nx * ny));
+    const int P = pp_zsolve_valid_lanes(nz, lanes) ? lanes : pp_zsolve_lanes(nz, cplx, (long)nx * ny);
     int ts = PP_Z_THREADS / P;
     if (systems >= 1 && (systems & (systems - 1)) == 0 && systems <= ts) {
         ts = systems;
@@ -936,6 +964,8 @@ void pp_zsolve_config_p(int nz, bool cplx, int nx, int lanes, int* TS, int* thre
     }
     while (ts > 1 && systems == 0 && pp_zsolve_smem_p(ts, nz, cplx, P) > 56 * 1024) ts >>= 1;
     while (ts > 1 && ts > nx) ts >>= 1;
+    // small grids: CTAs for every SM, in row segments of at least eight columns
+    while (ts > 8 && systems == 0 && ts * P > 32 && (long)ny * ((nx + ts - 1) / ts) < 296) ts >>= 1;
     *TS = ts;
     *threads = ts * P < 32 ? 32 : ts * P;
 }
@@ -955,8 +985,7 @@ cudaError_t pp_launch_zsolve(const PPZArgs& a0, bool cplx, cudaStream_t st)
 {
     if (a0.nz < 3 || a0.nz > pp_zsolve_max_nz(cplx, a0.data_fp32 != 0)) return cudaErrorInvalidValue;
     PPZArgs a = a0;
-    const bool large = pp_zsolve_large((long)a.nx * a.ny);
-    if (!pp_zsolve_valid_lanes(a.nz, a.P)) a.P = pp_zsolve_lanes(a.nz, cplx, large);
+    if (!pp_zsolve_valid_lanes(a.nz, a.P)) a.P = pp_zsolve_lanes(a.nz, cplx, (long)a.nx * a.ny);
     const int threads = a.TS * a.P < 32 ? 32 : a.TS * a.P;
     if (threads > PP_Z_THREADS) return cudaErrorInvalidValue;
     const size_t smem = zlayout(a.TS, a.nz, a.P, cplx, threads, a.data_fp32 != 0).bytes;
@@ -968,15 +997,13 @@ cudaError_t pp_launch_zsolve(const PPZArgs& a0, bool cplx, cudaStream_t st)
     const int rows = a.nz / a.P, rmax = (a.nz + a.P - 1) / a.P;
     const int mt = (a.nz % a.P == 0 && (rows == 8 || rows == 16 || ((rows == 10 || rows == 12) && cplx) ||
                                         ((rows == 20 || rows == 24 || rows == 32) && !cplx))) ? rows : 0;
-    int cap = 0;
-    if (!mt && large) {
-        if (cplx) cap = rmax <= 8 ? 8 : rmax <= 12 ? 12 : rmax <= 16 ? 16 : 0;
-        else cap = rmax <= 8 ? 8 : rmax <= 16 ? 16 : rmax <= 24 ? 24 : rmax <= 32 ? 32 : 0;
-    }
+    // (uneven counts: the next even capacity of the split path, or up to 8 rows)
+    const int most = cplx ? 19 : 34;
+    const int cap = mt || rmax > most ? 0 : rmax <= 8 ? 8 : (rmax + 1) / 2 * 2;
 #define PP_ZL(C, G, M, K) PP_ZLF((zsolve_kernel<C, G, M, K, false>))
-#define PP_ZLK(C, G, M, K, S)                                                                                   \
+#define PP_ZLK(C, G, M, K)                                                                                      \
     do {                                                                                                        \
-        PP_ZLF((split_kernel<C, G, M>()));                                                                     \
+        PP_ZLF((split_kernel<C, G, M, K>()));                                                                  \
     } while (0)
 #define PP_ZLF(KFN)                                                                                             \
     do {                                                                                                        \
@@ -990,17 +1017,26 @@ cudaError_t pp_launch_zsolve(const PPZArgs& a0, bool cplx, cudaStream_t st)
 #define PP_ZLM(C, G)                                  \
     do {                                              \
         if (mt == 8) PP_ZL(C, G, 8, false);           \
-        else if (mt == 16) PP_ZLK(C, G, 16, false, true); \
-        else if (mt == 32 && !C) PP_ZLK(C, G, (C ? 16 : 32), false, true); \
-        else if (mt == 24 && !C) PP_ZLK(C, G, (C ? 16 : 24), false, true); \
-        else if (mt == 12 && C) PP_ZLK(C, G, (C ? 12 : 16), false, true); \
-        else if (mt == 20 && !C) PP_ZLK(C, G, (C ? 16 : 20), false, true); \
-        else if (mt == 10 && C) PP_ZLK(C, G, (C ? 10 : 16), false, true); \
+        else if (mt == 16) PP_ZLK(C, G, 16, false);   \
+        else if (mt == 32 && !C) PP_ZLK(C, G, (C ? 16 : 32), false); \
+        else if (mt == 24 && !C) PP_ZLK(C, G, (C ? 16 : 24), false); \
+        else if (mt == 12 && C) PP_ZLK(C, G, (C ? 12 : 16), false); \
+        else if (mt == 20 && !C) PP_ZLK(C, G, (C ? 16 : 20), false); \
+        else if (mt == 10 && C) PP_ZLK(C, G, (C ? 10 : 16), false); \
         else if (cap == 8) PP_ZL(C, G, 8, true);      \
-        else if (cap == 12 && C) PP_ZL(C, G, (C ? 12 : 16), true); \
-        else if (cap == 16) PP_ZL(C, G, 16, true);    \
-        else if (cap == 24 && !C) PP_ZL(C, G, (C ? 16 : 24), true); \
-        else if (cap == 32 && !C) PP_ZL(C, G, (C ? 16 : 32), true); \
+        else if (cap == 10) PP_ZLK(C, G, 10, true);   \
+        else if (cap == 12) PP_ZLK(C, G, 12, true);   \
+        else if (cap == 14) PP_ZLK(C, G, 14, true);   \
+        else if (cap == 16) PP_ZLK(C, G, 16, true);   \
+        else if (cap == 18) PP_ZLK(C, G, 18, true);   \
+        else if (cap == 20) PP_ZLK(C, G, 20, true);   \
+        else if (cap == 22) PP_ZLK(C, G, (C ? 16 : 22), true); \
+        else if (cap == 24) PP_ZLK(C, G, (C ? 16 : 24), true); \
+        else if (cap == 26) PP_ZLK(C, G, (C ? 16 : 26), true); \
+        else if (cap == 28) PP_ZLK(C, G, (C ? 16 : 28), true); \
+        else if (cap == 30) PP_ZLK(C, G, (C ? 16 : 30), true); \
+        else if (cap == 32) PP_ZLK(C, G, (C ? 16 : 32), true); \
+        else if (cap == 34) PP_ZLK(C, G, (C ? 16 : 34), true); \
         else PP_ZL(C, G, 0, false);                   \
     } while (0)
     if (cplx && a.data_fp32) PP_ZLM(true, true);
