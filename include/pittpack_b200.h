@@ -274,7 +274,7 @@ typedef struct {
 typedef struct pp_batch_s* pp_batch;
 /* builds one handle per grid (options 'opt', or the defaults if null),
  * autotunes each size class once when 'autotune' is set, solves every grid
- * once and captures all solves into one graph whose 'branches' streams run
+ * once and captures all solves into one graph whose (at most) 'branches' streams run
  * concurrently; on the current device */
 int pp_batch_create(const pp_batch_item* items, int n, const pp_options* opt, int branches, int autotune,
                     pp_batch* out);

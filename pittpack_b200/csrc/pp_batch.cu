@@ -3,8 +3,9 @@
 //
 // The reference solves one grid per PencilDcmp object and launches every
 // step separately (src/pencilDcmp.cpp:5801-6430).  Here each grid keeps a
-// handle (plans, twiddles and workspaces resident on the device, zero-copy
-// bound to the caller's RHS and solution buffers), the launch shape of each
+// handle (plans and twiddles resident on the device, zero-copy bound to the
+// caller's RHS and solution buffers, the workspaces shared by the grids of a
+// branch), the launch shape of each
 // size class is chosen once by the autotuner, and the solves of all grids are
 // captured into one graph whose branches run concurrently, so that small grids
 // fill the GPU together and the whole batch costs one graph launch.
@@ -14,11 +15,21 @@
 #include <tuple>
 #include <vector>
 
+#include <algorithm>
+
 #include "../../include/pittpack_b200.h"
+#include "pp_kernels.h"
 
 struct pp_batch_s {
     int device = 0;
     std::vector<pp_handle> handles;
+    // per branch, one workspace that its grids take in turn (two spectra, and
+    // the FP32 residual of the refined solve): what a grid leaves in L2 is
+    // overwritten there by the next one instead of going to memory
+    struct Workspace {
+        void* p[3] = {nullptr, nullptr, nullptr};
+    };
+    std::vector<Workspace> work;
     std::vector<cudaStream_t> branches;
     cudaStream_t cap = nullptr;
     cudaGraph_t graph = nullptr;
@@ -35,21 +46,65 @@ void batch_free(pp_batch_s* b)
     if (b->graph) cudaGraphDestroy(b->graph);
     // the handles name the branch streams: release them first
     for (auto h : b->handles) pp_destroy(h);
+    for (auto& w : b->work)
+        for (void* q : w.p)
+            if (q) cudaFree(q);
     for (auto s : b->branches) cudaStreamDestroy(s);
     if (b->cap) cudaStreamDestroy(b->cap);
     delete b;
 }
 
-// one handle per grid, tuned per size class, solved once outside the capture
-int build_handles(pp_batch_s* b, const pp_batch_item* items, int n, const pp_options* opt, int autotune)
+// How many grids run at once, at most 'branches': as many as keep their spectra
+// in three quarters of L2 together (right-hand sides and solutions pass through
+// the rest).  A grid's passes hand the two spectra from one to the next through
+// L2; past its capacity every pass goes to memory and back (48 grids of 32 ..
+// 192 points an edge, 126 MB of L2: 1.95 ms at 3 and 4 branches, 2.1 at 5, 2.40
+// at 8, 2.44 at 16, 2.07 at 2, 2.53 at 1).  Larger grids still run two at a time,
+// so that one fills the other's tails.
+int branches_in_l2(const pp_batch_item* items, int n, bool refined, int branches)
 {
+    int dev = 0, l2 = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess ||
+        l2 <= 0)
+        return branches;
+    double bytes = 0.0;
+    for (int i = 0; i < n; ++i) {
+        // two real spectra (half spectra of a periodic x as much), the second one
+        // complex for a periodic y alone; refined: FP32 spectra and residual, u
+        if (items[i].nx <= 0 || items[i].ny <= 0 || items[i].nz <= 0) continue;  // rejected later
+        const bool wide = items[i].bc[2] == 'P' && items[i].bc[0] != 'P';
+        bytes += (refined ? 20.0 : wide ? 24.0 : 16.0) * items[i].nx * (double)items[i].ny * items[i].nz;
+    }
+    const double fit = bytes > 0 ? 0.75 * l2 * n / bytes : branches;
+    return fit >= branches ? branches : std::min(branches, std::max(2, (int)fit));
+}
+
+// one handle per grid, tuned per size class, solved once outside the capture
+int build_handles(pp_batch_s* b, const pp_batch_item* items, int n, const pp_options* opt, int branches, int autotune)
+{
+    const bool refined = opt && opt->precision == PP_PRECISION_MIXED;
+    b->work.resize(branches);
+    for (int k = 0; k < branches; ++k) {
+        size_t bytes = 0;
+        for (int i = k; i < n; i += branches) {
+            const pp_batch_item& it = items[i];
+            if (it.nx > 0 && it.ny > 0 && it.nz > 0) bytes = std::max(bytes, pp_spectrum_bytes(it.nx, it.ny, it.nz));
+        }
+        const size_t want[3] = {bytes, bytes, refined ? bytes / 4 : 0};
+        for (int q = 0; q < 3; ++q)
+            if (want[q] && cudaMalloc(&b->work[k].p[q], want[q]) != cudaSuccess) {
+                cudaGetLastError();
+                return PP_ALLOCATION_FAIL;
+            }
+    }
     // tuned launch shape per size class (nx, ny, nz, boundary letters)
     std::map<std::tuple<int, int, int, std::string>, pp_tuning> tuned;
     int rc = PP_SUCCESS;
     for (int i = 0; i < n && rc == PP_SUCCESS; ++i) {
         const pp_batch_item& it = items[i];
         pp_handle h = nullptr;
-        if ((rc = pp_create(it.nx, it.ny, it.nz, &h)) != PP_SUCCESS) break;
+        void* const* w = b->work[i % branches].p;
+        if ((rc = pp_create_lent(it.nx, it.ny, it.nz, w[0], w[1], w[2], &h)) != PP_SUCCESS) break;
         b->handles.push_back(h);
         if ((rc = pp_set_box(h, it.box)) != PP_SUCCESS) break;
         if ((rc = pp_assign_boundary(h, it.bc)) != PP_SUCCESS) break;
@@ -88,7 +143,8 @@ extern "C" int pp_batch_create(const pp_batch_item* items, int n, const pp_optio
     pp_batch_s* b = new (std::nothrow) pp_batch_s;
     if (!b) return PP_ALLOCATION_FAIL;
     cudaGetDevice(&b->device);
-    int rc = build_handles(b, items, n, opt, autotune);
+    branches = branches_in_l2(items, n, opt && opt->precision == PP_PRECISION_MIXED, branches);
+    int rc = build_handles(b, items, n, opt, branches, autotune);
     if (rc != PP_SUCCESS) {
         batch_free(b);
         return rc;

@@ -240,3 +240,13 @@ struct PPZRefArgs {
 };
 bool pp_zsolve_ref_defined(int method, int nz, int zlo, int zhi);
 cudaError_t pp_launch_zsolve_ref(const PPZRefArgs& a, cudaStream_t st);
+
+struct pp_solver_s;
+// bytes of each of a handle's grid-sized buffers
+size_t pp_spectrum_bytes(int nx, int ny, int nz);
+// a handle (pp_destroy frees it) that works in its caller's memory: the two
+// spectrum buffers, and for the refined solve a quarter as much for the FP32
+// residual (null otherwise).  The caller binds the right-hand side and the
+// solution (pp_bind_device_buffers) before a solve, keeps the memory longer than
+// the handle, and runs handles that share it one after the other.
+int pp_create_lent(int nx, int ny, int nz, void* spec_a, void* spec_b, void* work, pp_solver_s** out);

@@ -42,6 +42,7 @@ bool radix_plan(int n, std::vector<int>& r)
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    bool lent = false;  // memory of another owner (a batch's shared workspace)
     cudaError_t alloc(size_t b)
     {
         free();
@@ -50,11 +51,19 @@ struct DevBuf {
         else p = nullptr;
         return e;
     }
+    void borrow(void* q, size_t b)
+    {
+        free();
+        p = q;
+        bytes = b;
+        lent = true;
+    }
     void free()
     {
-        if (p) cudaFree(p);
+        if (p && !lent) cudaFree(p);
         p = nullptr;
         bytes = 0;
+        lent = false;
     }
     template <typename T>
     T* as() const { return static_cast<T*>(p); }
@@ -1163,10 +1172,9 @@ int pp_default_options(pp_options* opt)
     return PP_SUCCESS;
 }
 
-int pp_create(int nx, int ny, int nz, pp_handle* out)
+// a new handle without its grid buffers; PP_SUCCESS or what pp_create returns
+static int new_handle(int nx, int ny, int nz, pp_solver_s** out)
 {
-    if (!out) return PP_INPUT_ARGS;
-    *out = nullptr;
     if (nx < 2 || ny < 2 || nz < 3) return PP_INPUT_ARGS;
     if (nz > pp_zsolve_max_nz(false, false)) return PP_UNSUPPORTED;
     int ndev = 0;
@@ -1178,10 +1186,25 @@ int pp_create(int nx, int ny, int nz, pp_handle* out)
     h->nz = nz;
     cudaGetDevice(&h->device);
     pp_default_options(&h->opt);
-    const size_t n = (size_t)nx * ny * nz;
-    if (h->rhs.alloc(2 * n * sizeof(double)) != cudaSuccess || h->bufA.alloc(2 * n * sizeof(double)) != cudaSuccess ||
-        h->bufB.alloc(2 * n * sizeof(double)) != cudaSuccess || h->out.alloc(2 * n * sizeof(double)) != cudaSuccess ||
-        h->errc.alloc(sizeof(int)) != cudaSuccess || cudaMemset(h->errc.p, 0, sizeof(int)) != cudaSuccess) {
+    if (h->errc.alloc(sizeof(int)) != cudaSuccess || cudaMemset(h->errc.p, 0, sizeof(int)) != cudaSuccess) {
+        h->errc.free();
+        cudaGetLastError();
+        delete h;
+        return PP_ALLOCATION_FAIL;
+    }
+    *out = h;
+    return PP_SUCCESS;
+}
+
+int pp_create(int nx, int ny, int nz, pp_handle* out)
+{
+    if (!out) return PP_INPUT_ARGS;
+    *out = nullptr;
+    pp_solver_s* h = nullptr;
+    if (const int rc = new_handle(nx, ny, nz, &h)) return rc;
+    const size_t bytes = pp_spectrum_bytes(nx, ny, nz);
+    if (h->rhs.alloc(bytes) != cudaSuccess || h->bufA.alloc(bytes) != cudaSuccess ||
+        h->bufB.alloc(bytes) != cudaSuccess || h->out.alloc(bytes) != cudaSuccess) {
         // release what did fit (the buffers have no destructor)
         h->rhs.free();
         h->bufA.free();
@@ -1893,3 +1916,18 @@ int pp_autotune(pp_handle h, int reps, pp_tuning* chosen, double* best_ms)
 }
 
 }  // extern "C"
+
+size_t pp_spectrum_bytes(int nx, int ny, int nz) { return 2 * sizeof(double) * (size_t)nx * ny * nz; }
+
+int pp_create_lent(int nx, int ny, int nz, void* spec_a, void* spec_b, void* work, pp_solver_s** out)
+{
+    *out = nullptr;
+    pp_solver_s* h = nullptr;
+    if (const int rc = new_handle(nx, ny, nz, &h)) return rc;
+    const size_t bytes = pp_spectrum_bytes(nx, ny, nz);
+    h->bufA.borrow(spec_a, bytes);
+    h->bufB.borrow(spec_b, bytes);
+    h->out.borrow(work, work ? bytes / 4 : 0);
+    *out = h;
+    return PP_SUCCESS;
+}
