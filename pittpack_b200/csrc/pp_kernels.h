@@ -69,6 +69,31 @@ struct PPLinePassArgs {
     int* err;
 };
 
+// The run-time planned transform pass (pp_mr.cuh): lengths whose FFT factors
+// into 2, 3, 5, 7, 11 and 13; passed to the kernel by value
+#define PP_MR_MAXPASS 6
+struct PPMrPlan {
+    int m;                          // FFT points a line (0: no such plan)
+    int L, lgl;                     // FFT lines a CTA (a power of two)
+    int npass;
+    int radix[PP_MR_MAXPASS];
+    unsigned magic[PP_MR_MAXPASS];  // division by the span of each pass
+    int threads;
+};
+// the plan of a direction (half: its periodic half spectra); false where it has none
+bool pp_mr_plan(int n, int kind, bool half, PPMrPlan* p);
+// data lines per CTA tile
+int pp_mr_lines(int n, int kind, const PPMrPlan& p);
+// one pass (a.tw and a.cs2 in its precision, strides and output strides set)
+cudaError_t pp_mr_line_pass(PPLinePassArgs a, const PPMrPlan& p, bool inverse, bool strided, bool in_cplx,
+                            bool out_cplx, bool fp32, cudaStream_t st);
+cudaError_t pp_launch_mr_real_f64(const PPLinePassArgs& a, const PPMrPlan& p, bool inverse, bool strided, cudaStream_t st);
+cudaError_t pp_launch_mr_real_f32(const PPLinePassArgs& a, const PPMrPlan& p, bool inverse, bool strided, cudaStream_t st);
+cudaError_t pp_launch_mr_periodic_f64(const PPLinePassArgs& a, const PPMrPlan& p, bool inverse, bool strided,
+                                      cudaStream_t st);
+cudaError_t pp_launch_mr_periodic_f32(const PPLinePassArgs& a, const PPMrPlan& p, bool inverse, bool strided,
+                                      cudaStream_t st);
+
 // shared memory of the generic kernel: two buffers of L lines of nfft complex
 // points in FP64, or in FP32 (fp32)
 size_t pp_line_pass_smem(int L, int nfft, bool fp32 = false);
@@ -111,10 +136,6 @@ cudaError_t pp_launch_long_line_pass(const PPLinePassArgs& a, const PPLongPlan& 
 int pp_lp2_lpc(int n);
 template <typename Real, typename TI, typename TO>
 cudaError_t pp_launch_line_pass_pow2(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st);
-// the same kernel for the lengths 3 2^k (48 .. 1536), 5 2^k (80 .. 1280),
-// 9 2^k (144 .. 1152) and 15 2^k (240 .. 960):
-// complex FFT lines per CTA (0 = not covered), and the FP64 / FP32 launches
-int pp_lpm_lpc(int n);
 // the real families and the periodic half spectra through a complex FFT of
 // half the length (pp_rhalf.cuh): data lines per CTA tile (0 = not covered),
 // whether a pass takes that kernel, and the pass (a.tw and a.cs2 in its
@@ -124,11 +145,6 @@ bool pp_rh_covers(const PPLinePassArgs& a, bool inverse, bool strided, bool out_
 cudaError_t pp_rh_line_pass(PPLinePassArgs a, bool inverse, bool strided, bool in_cplx, bool out_cplx, bool fp32,
                             cudaStream_t st);
 cudaError_t pp_launch_line_pass_rh_f32(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st);
-cudaError_t pp_launch_line_pass_mixed(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st);
-cudaError_t pp_launch_line_pass_mixed_f32(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st);
-// 9 2^k and 15 2^k (144 .. 1152), called by the two above
-cudaError_t pp_launch_line_pass_mixed915(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st);
-cudaError_t pp_launch_line_pass_mixed915_f32(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st);
 // every other length (pp_fft_plan); fp32: the FP32 kernel, twiddles from a.tw and
 // a.cs2 (FP64: a.fft.tw and a.cs), with the refinement epilogue when a.acc is set
 cudaError_t pp_launch_line_pass(const PPLinePassArgs& a, bool inverse, bool strided, bool in_cplx, bool out_cplx,

@@ -1,12 +1,10 @@
-// Transform pass for line lengths N = m 2^k (m = 1, 3, 5, 9, 15; the FFT's
-// power-of-two factor at least 8; the real families and half spectra of
-// N = 32 .. 1024, m = 1, take pp_rhalf.cuh): the same four passes and the same
+// Transform pass for line lengths N = 16 .. 2048, powers of two (the real
+// families and half spectra of N = 32 .. 1024 take pp_rhalf.cuh, so that those
+// lengths are here for complex lines): the same four passes and the same
 // per-family pre/post-processing as pp_linepass.cu (see the reference
 // citations there), built on the register-resident FFT of pp_fftreg.cuh and
 // specialised at compile time on the length and the boundary family, so that
-// reorders, signs and twiddle selection cost no run-time branches.  The
-// power-of-two factor runs as register passes; an odd factor m > 1 as one
-// final Stockham pass of radix m and span 2^k in shared memory.
+// reorders, signs and twiddle selection cost no run-time branches.
 //
 //   FFT family (P-P): LPC complex lines per CTA, one FFT of N each.
 //   DCT-II/III, DST-II/III (N-N, D-D): 2 LPC real lines per CTA, packed two
@@ -60,46 +58,6 @@ struct Vec2<float> {
 };
 
 PP_D int mk_pos(int e, int n) { return (e & 1) ? (n - 1 - (e >> 1)) : (e >> 1); }
-
-// R-point DFT in registers, R = 3 or 5 (pp_fft.cuh)
-template <int SIGN, int R, typename C>
-PP_D void small_dft(C* v)
-{
-    if constexpr (R == 3) dft3<SIGN>(v);
-    else dft5<SIGN>(v);
-}
-
-// MM = A B point DFT by one Cooley-Tukey step: n = B n1 + n2, k = k1 + A k2;
-// A-point DFTs over n1, twiddles W_MM^{n2 k1}, B-point DFTs over n2.  W_MM^x
-// is taken from the FFT's own table as tw[x * stride] (stride = NF / MM).
-template <int SIGN, int A, int B, typename C>
-PP_D void dft_ct(C* v, const C* __restrict__ tw, int stride)
-{
-    C y[B][A];
-#pragma unroll
-    for (int n2 = 0; n2 < B; ++n2) {
-#pragma unroll
-        for (int n1 = 0; n1 < A; ++n1) y[n2][n1] = v[B * n1 + n2];
-        small_dft<SIGN, A>(y[n2]);
-    }
-#pragma unroll
-    for (int n2 = 1; n2 < B; ++n2)
-#pragma unroll
-        for (int k1 = 1; k1 < A; ++k1) {
-            C w = __ldg(&tw[n2 * k1 * stride]);
-            if (SIGN > 0) w.y = -w.y;
-            y[n2][k1] = c_mul(y[n2][k1], w);
-        }
-#pragma unroll
-    for (int k1 = 0; k1 < A; ++k1) {
-        C z[B];
-#pragma unroll
-        for (int n2 = 0; n2 < B; ++n2) z[n2] = y[n2][k1];
-        small_dft<SIGN, B>(z);
-#pragma unroll
-        for (int k2 = 0; k2 < B; ++k2) v[k1 + A * k2] = z[k2];
-    }
-}
 
 PP_D double lift_at(const PPLift& L, int i, int j, int k, int nx, int ny, int nz)
 {
@@ -355,11 +313,8 @@ __device__ __forceinline__ void lp2_body(const PPLinePassArgs& a)
     // radix 8 first: register q holds point m = t + q N/8 (t < N/8), so the
     // half of the line it falls in is known from q at compile time
     constexpr int NF = Q4 ? N / 2 : N;  // FFT length
-    constexpr int MF = rp_pow2_part(NF);  // its power-of-two factor (register passes)
-    constexpr int MM = NF / MF;           // and its odd factor (one radix-MM pass)
-    static_assert(MM == 1 || MM == 3 || MM == 5 || MM == 9 || MM == 15, "FFT length 2^k, 3 2^k, 5 2^k, 9 2^k or 15 2^k");
     constexpr int TPL = NF / 8;         // threads per FFT line
-    static_assert(rp_radix(MF, 0) == 8, "the first pass is radix 8");
+    static_assert(rp_radix(NF, 0) == 8, "the first pass is radix 8");
     static_assert(!(FAM == F_DST2 && INVERSE) || TPL % 2 == 0, "the DST-III sign uses the parity of t");
     const int fl = tid / TPL;           // FFT line of this thread
     const int t = tid - fl * TPL;
@@ -464,48 +419,10 @@ __device__ __forceinline__ void lp2_body(const PPLinePassArgs& a)
     // ---- 3. FFT (its first exchange starts with a barrier, so the raw tile
     //         that aliases the line buffers is no longer needed) ----------------------
     constexpr int FS = (INVERSE && !Q4) ? +1 : -1;
-    rp_fft<FS, NF, MF>(v, line, t, tw);
+    rp_fft<FS, NF>(v, line, t, tw);
     __syncthreads();  // all reads of the last exchange are done
-    if constexpr (MM == 1) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) line[rp_pad(rp_out_index<NF>(t, j))] = v[j];
-    } else {
-        // Stockham output of the last register pass, then the final pass of
-        // radix MM and span MF, in place: butterfly j < MF reads points
-        // j + q MF, multiplies point q by W_NF^{q j} and writes output q to
-        // j + q MF (natural order)
-        constexpr int NPM = rp_npass(MF);
-        rp_scatter<NF, rp_radix(MF, NPM - 1), rp_ns(MF, NPM - 1)>(v, line, t);
-        __syncthreads();
-        constexpr int NB = (MF + TPL - 1) / TPL;  // butterflies of this thread, at most
-        C u[NB][MM];
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const int j = t + b * TPL;
-            if (j < MF) {
-#pragma unroll
-                for (int q = 0; q < MM; ++q) u[b][q] = line[rp_pad(j + q * MF)];
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const int j = t + b * TPL;
-            if (j < MF) {
-#pragma unroll
-                for (int q = 1; q < MM; ++q) {
-                    C w = __ldg(&tw[q * j]);
-                    if (FS > 0) w.y = -w.y;
-                    u[b][q] = c_mul(u[b][q], w);
-                }
-                if constexpr (MM == 3 || MM == 5) small_dft<FS, MM>(u[b]);
-                else if constexpr (MM == 9) dft_ct<FS, 3, 3>(u[b], tw, MF);
-                else dft_ct<FS, 5, 3>(u[b], tw, MF);
-#pragma unroll
-                for (int q = 0; q < MM; ++q) line[rp_pad(j + q * MF)] = u[b][q];
-            }
-        }
-    }
+    for (int j = 0; j < 8; ++j) line[rp_pad(rp_out_index<NF>(t, j))] = v[j];
     __syncthreads();
 
     // ---- 4. post-processing and stores ------------------------------------------------
@@ -699,18 +616,8 @@ __device__ __forceinline__ void lp2_body(const PPLinePassArgs& a)
     }
 }
 
-// the power-of-two lengths, and (with a register bound that leaves room for
-// one more CTA per SM) the lengths with an odd factor, whose final radix-m
-// pass holds up to three butterflies per thread.  The second argument of
-// __launch_bounds__ is what bounds the registers.
-constexpr int lpm_min_blocks(int nt) { return 65536 / (84 * nt) > 1 ? 65536 / (84 * nt) : 1; }
 template <typename Real, int N, int LPC, int FAM, bool INVERSE, bool STRIDED>
 __global__ void __launch_bounds__(LPC * N / 8) lp2_kernel(PPLinePassArgs a)
-{
-    lp2_body<Real, N, LPC, FAM, INVERSE, STRIDED>(a);
-}
-template <typename Real, int N, int LPC, int FAM, bool INVERSE, bool STRIDED>
-__global__ void __launch_bounds__(LPC * N / 8, lpm_min_blocks(LPC * N / 8)) lpm_kernel(PPLinePassArgs a)
 {
     lp2_body<Real, N, LPC, FAM, INVERSE, STRIDED>(a);
 }
@@ -726,8 +633,7 @@ constexpr auto pass_kernel()
 {
     if constexpr (N == 512 && FAM == F_FFT && std::is_same<Real, double>::value)
         return lp2b_kernel<Real, N, LPC, FAM, INVERSE, STRIDED>;
-    else if constexpr ((N & (N - 1)) == 0) return lp2_kernel<Real, N, LPC, FAM, INVERSE, STRIDED>;
-    else return lpm_kernel<Real, N, LPC, FAM, INVERSE, STRIDED>;
+    else return lp2_kernel<Real, N, LPC, FAM, INVERSE, STRIDED>;
 }
 
 template <typename Real, int N, int LPC, int FAM>
@@ -765,7 +671,7 @@ cudaError_t launch_half(const PPLinePassArgs& a, cudaStream_t st)
 template <typename Real, int N, int LPC>
 cudaError_t launch_n(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st)
 {
-    if constexpr (N >= 32 && N <= 1024 && (N & (N - 1)) == 0) {
+    if constexpr (N >= 32 && N <= 1024) {
         // the real families and the half spectra of these lengths: pp_rhalf.cuh
         return a.kind == PP_KIND_FFT && !a.half ? launch_fam<Real, N, LPC, F_FFT>(a, inverse, strided, st)
                                                 : cudaErrorInvalidValue;
@@ -812,71 +718,6 @@ cudaError_t launch(const PPLinePassArgs& a, bool inverse, bool strided, cudaStre
     case 512: return launch_n<Real, 512, 4>(a, inverse, strided, st);
     case 1024: return launch_n<Real, 1024, 2>(a, inverse, strided, st);
     case 2048: return launch_n<Real, 2048, 1>(a, inverse, strided, st);
-    default: return cudaErrorInvalidValue;
-    }
-}
-
-// lines per CTA for the lengths m 2^k, m = 3, 5, 9, 15, with 2^k >= 16 so
-// that the quarter-wave families' half-length FFT still starts with a
-// radix-8 register pass (the register passes take the power-of-two factor,
-// one shared-memory pass the odd one); 0 if the length has no such kernel
-inline int lpm_of(int n)
-{
-    switch (n) {
-    case 48: return 8;
-    case 80: return 8;
-    case 96: return 8;
-    case 144: return 8;
-    case 160: return 4;
-    case 192: return 4;
-    case 240: return 4;
-    case 288: return 4;
-    case 320: return 4;
-    case 384: return 4;
-    case 480: return 2;
-    case 576: return 2;
-    case 640: return 2;
-    case 768: return 2;
-    case 960: return 1;
-    case 1152: return 1;
-    case 1280: return 1;
-    case 1536: return 1;
-    default: return 0;
-    }
-}
-inline bool lpm_odd9or15(int n) { return n == 144 || n == 240 || n == 288 || n == 480 || n == 576 || n == 960 || n == 1152; }
-
-// the odd factors 9 and 15 (their own translation units)
-template <typename Real>
-cudaError_t launch_mixed915(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st)
-{
-    switch (a.n) {
-    case 144: return launch_n<Real, 144, 8>(a, inverse, strided, st);
-    case 240: return launch_n<Real, 240, 4>(a, inverse, strided, st);
-    case 288: return launch_n<Real, 288, 4>(a, inverse, strided, st);
-    case 480: return launch_n<Real, 480, 2>(a, inverse, strided, st);
-    case 576: return launch_n<Real, 576, 2>(a, inverse, strided, st);
-    case 960: return launch_n<Real, 960, 1>(a, inverse, strided, st);
-    case 1152: return launch_n<Real, 1152, 1>(a, inverse, strided, st);
-    default: return cudaErrorInvalidValue;
-    }
-}
-
-template <typename Real>
-cudaError_t launch_mixed(const PPLinePassArgs& a, bool inverse, bool strided, cudaStream_t st)
-{
-    switch (a.n) {
-    case 48: return launch_n<Real, 48, 8>(a, inverse, strided, st);
-    case 80: return launch_n<Real, 80, 8>(a, inverse, strided, st);
-    case 96: return launch_n<Real, 96, 8>(a, inverse, strided, st);
-    case 160: return launch_n<Real, 160, 4>(a, inverse, strided, st);
-    case 192: return launch_n<Real, 192, 4>(a, inverse, strided, st);
-    case 320: return launch_n<Real, 320, 4>(a, inverse, strided, st);
-    case 384: return launch_n<Real, 384, 4>(a, inverse, strided, st);
-    case 640: return launch_n<Real, 640, 2>(a, inverse, strided, st);
-    case 768: return launch_n<Real, 768, 2>(a, inverse, strided, st);
-    case 1280: return launch_n<Real, 1280, 1>(a, inverse, strided, st);
-    case 1536: return launch_n<Real, 1536, 1>(a, inverse, strided, st);
     default: return cudaErrorInvalidValue;
     }
 }

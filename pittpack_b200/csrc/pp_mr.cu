@@ -1,0 +1,74 @@
+// Host side of the run-time planned transform pass (pp_mr.cuh): the radices,
+// lines and threads of a length, and one pass in either precision.
+#include "pp_mr.cuh"
+cudaError_t pp_launch_mr_ct_a_f64(const PPLinePassArgs&, const PPMrPlan&, bool, bool, cudaStream_t);
+cudaError_t pp_launch_mr_ct_a_f32(const PPLinePassArgs&, const PPMrPlan&, bool, bool, cudaStream_t);
+cudaError_t pp_launch_mr_ct_b_f64(const PPLinePassArgs&, const PPMrPlan&, bool, bool, cudaStream_t);
+cudaError_t pp_launch_mr_ct_b_f32(const PPLinePassArgs&, const PPMrPlan&, bool, bool, cudaStream_t);
+cudaError_t pp_launch_mr_ct_c_f64(const PPLinePassArgs&, const PPMrPlan&, bool, bool, cudaStream_t);
+cudaError_t pp_launch_mr_ct_c_f32(const PPLinePassArgs&, const PPMrPlan&, bool, bool, cudaStream_t);
+cudaError_t pp_launch_mr_ct_d_f64(const PPLinePassArgs&, const PPMrPlan&, bool, bool, cudaStream_t);
+cudaError_t pp_launch_mr_ct_d_f32(const PPLinePassArgs&, const PPMrPlan&, bool, bool, cudaStream_t);
+cudaError_t pp_launch_mr_ct_e_f64(const PPLinePassArgs&, const PPMrPlan&, bool, bool, cudaStream_t);
+cudaError_t pp_launch_mr_ct_e_f32(const PPLinePassArgs&, const PPMrPlan&, bool, bool, cudaStream_t);
+
+namespace {
+
+// the instances planned at compile time, by ranges of lengths; within a range
+// the lengths without one answer cudaErrorInvalidValue
+using CtLaunch = cudaError_t (*)(const PPLinePassArgs&, const PPMrPlan&, bool, bool, cudaStream_t);
+struct CtRange {
+    int lo, hi;
+    CtLaunch f64, f32;
+};
+const CtRange kCt[] = {
+    {40, 120, pp_launch_mr_ct_a_f64, pp_launch_mr_ct_a_f32},
+    {144, 250, pp_launch_mr_ct_b_f64, pp_launch_mr_ct_b_f32},
+    {270, 450, pp_launch_mr_ct_c_f64, pp_launch_mr_ct_c_f32},
+    {480, 768, pp_launch_mr_ct_d_f64, pp_launch_mr_ct_d_f32},
+    {800, 1536, pp_launch_mr_ct_e_f64, pp_launch_mr_ct_e_f32},
+};
+
+}  // namespace
+
+bool pp_mr_plan(int n, int kind, bool half, PPMrPlan* p)
+{
+    *p = PPMrPlan{};
+    const bool odd = n & 1;
+    if ((half || pp_kind_is_quarter(kind)) && odd) return false;
+    *p = pp_mr::make_plan((half || (kind != PP_KIND_FFT && !odd)) ? n / 2 : n);
+    return p->m > 0;
+}
+
+int pp_mr_lines(int n, int kind, const PPMrPlan& p)
+{
+    // real lines of odd length go two to an FFT line
+    return (kind != PP_KIND_FFT && (n & 1)) ? 2 * p.L : p.L;
+}
+
+cudaError_t pp_mr_line_pass(PPLinePassArgs a, const PPMrPlan& p, bool inverse, bool strided, bool in_cplx,
+                            bool out_cplx, bool fp32, cudaStream_t st)
+{
+    const size_t es = fp32 ? sizeof(float) : sizeof(double);
+    const bool own = a.o_elem_stride != 0;
+    a.in_cplx = in_cplx;
+    a.out_cplx = out_cplx;
+    // pairs of reals in, pairs of reals or (the solution P) of complex points out
+    auto whole = [](const void* q, long s1, long s2, size_t elem, size_t w) {
+        return reinterpret_cast<uintptr_t>(q) % w == 0 && ((size_t)s1 * elem) % w == 0 && ((size_t)s2 * elem) % w == 0;
+    };
+    a.vec16 = !strided && !in_cplx && whole(a.src, a.line_stride, a.plane_stride, es, 2 * es);
+    a.vec_out = !strided && whole(a.dst, own ? a.o_line_stride : a.line_stride, own ? a.o_plane_stride : a.plane_stride,
+                                  (out_cplx ? 2 : 1) * es, (inverse ? 4 : 2) * es);
+    a.L = pp_mr_lines(a.n, a.kind, p);
+    a.tiles_per_plane = (a.nlines + a.L - 1) / a.L;
+    for (const CtRange& c : kCt)
+        if (a.n >= c.lo && a.n <= c.hi) {
+            const cudaError_t e = (fp32 ? c.f32 : c.f64)(a, p, inverse, strided, st);
+            if (e != cudaErrorInvalidValue) return e;
+        }
+    if (a.kind == PP_KIND_FFT)
+        return fp32 ? pp_launch_mr_periodic_f32(a, p, inverse, strided, st)
+                    : pp_launch_mr_periodic_f64(a, p, inverse, strided, st);
+    return fp32 ? pp_launch_mr_real_f32(a, p, inverse, strided, st) : pp_launch_mr_real_f64(a, p, inverse, strided, st);
+}

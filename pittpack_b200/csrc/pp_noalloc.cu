@@ -83,7 +83,7 @@ int na_dir(NaDir& d, int n, int kind)
     d.kind = kind;
     d.nf = pp_fft_len(n, kind);
     if (!pp_fft_plan(d.nf, &d.fft)) return PP_UNSUPPORTED;
-    if (pp_lp2_lpc(n) == 0 && pp_lpm_lpc(n) == 0 && pp_line_pass_smem(1, d.nf) > 227 * 1024) return PP_UNSUPPORTED;
+    if (pp_lp2_lpc(n) == 0 && pp_line_pass_smem(1, d.nf) > 227 * 1024) return PP_UNSUPPORTED;
     return PP_SUCCESS;
 }
 
@@ -212,7 +212,7 @@ cudaError_t na_line_pass(PPLinePassArgs a, const NaDir& d, const double2* tw, co
         a.cs2 = cs;
         return pp_rh_line_pass(a, inverse, strided, in_cplx, out_cplx, false, st);
     }
-    const int lpc2 = pp_lp2_lpc(d.n), lpc = lpc2 ? lpc2 : pp_lpm_lpc(d.n);
+    const int lpc = pp_lp2_lpc(d.n);
     if (lpc > 0) {
         a.tw = tw;
         a.cs2 = cs;
@@ -221,8 +221,13 @@ cudaError_t na_line_pass(PPLinePassArgs a, const NaDir& d, const double2* tw, co
         const int dl = d.kind == PP_KIND_FFT ? lpc : 2 * lpc;
         a.L = dl;
         a.tiles_per_plane = (a.nlines + dl - 1) / dl;
-        return lpc2 ? pp_launch_line_pass_pow2<double, double, double>(a, inverse, strided, st)
-                    : pp_launch_line_pass_mixed(a, inverse, strided, st);
+        return pp_launch_line_pass_pow2<double, double, double>(a, inverse, strided, st);
+    }
+    PPMrPlan mr;
+    if ((d.kind == PP_KIND_FFT || !out_cplx || (inverse && !strided)) && pp_mr_plan(d.n, d.kind, false, &mr)) {
+        a.tw = tw;
+        a.cs2 = cs;
+        return pp_mr_line_pass(a, mr, inverse, strided, in_cplx, out_cplx, false, st);
     }
     int L = 16;
     while (L > 1 && pp_line_pass_smem(L, d.fft.n) > 64 * 1024) L >>= 1;

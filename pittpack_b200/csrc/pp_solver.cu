@@ -73,6 +73,7 @@ struct DevBuf {
 struct DirTables {
     int n = 0, kind = -1;
     PPFftPlan fft{};
+    PPMrPlan mr{}, mrh{};  // run-time planned passes of the lines, and of half spectra (m = 0: none)
     DevBuf tw;   // FFT twiddles of length fft.n
     DevBuf cs;   // family pre/post twiddles
     DevBuf eig;  // -2 + 2 cos((k + num) f / (n + den)), k < n
@@ -291,6 +292,7 @@ int build_dir(pp_solver_s* h, DirTables& t, int n, int kind)
     // shared memory: longer lines, outside the register kernels, run the
     // four-step FFT through global memory (pp_longline.cu) where nf splits
     t.n1 = t.n2 = t.M = 0;
+    t.mr = t.mrh = PPMrPlan{};
     // lines past one generic-kernel tile, and lengths whose largest prime
     // factor p makes the generic kernel's direct p-point pass (p^2 work per
     // butterfly) slower than the chirp z-transform: measured on 64 x 64
@@ -298,7 +300,7 @@ int build_dir(pp_solver_s* h, DirTables& t, int n, int kind)
     // 2.28 / 0.62, p = 1031 937 / 3.6, p = 4099 29500 / 14.4
     const bool long_line = pp_line_pass_smem(1, nf) > 227 * 1024;
     const bool big_prime = largest_prime_factor(nf) >= PP_CHIRP_MIN_PRIME;
-    if (pp_lp2_lpc(n) == 0 && pp_lpm_lpc(n) == 0 && (long_line || big_prime)) {
+    if (pp_lp2_lpc(n) == 0 && (long_line || big_prime)) {
         // four-step where nf splits into two tiles, else the chirp z-transform
         int n1 = 0, n2 = 0, M = 0;
         if ((big_prime || !pp_long_split(nf, &n1, &n2)) && !pp_bluestein_split(nf, &M, &n1, &n2)) return PP_UNSUPPORTED;
@@ -316,6 +318,10 @@ int build_dir(pp_solver_s* h, DirTables& t, int n, int kind)
         }
         t.f1.tw = t.tw1.as<double2>();
         t.f2.tw = t.tw2.as<double2>();
+    }
+    if (t.n1 == 0) {
+        pp_mr_plan(n, kind, false, &t.mr);
+        if (kind == PP_KIND_FFT) pp_mr_plan(n, kind, true, &t.mrh);
     }
     t.fft.n = nf;
     t.fft.npass = (int)r.size();
@@ -552,7 +558,8 @@ int runs_aligned16(const PPLinePassArgs& a, bool strided, size_t elem_bytes, int
            ((size_t)dl * ts * elem_bytes) % 16 == 0;
 }
 
-// one transform pass: the register-resident kernel for power-of-two lengths,
+// one transform pass: the register-resident kernels for power-of-two lengths, the
+// planned kernel for lengths that factor into 2 .. 13, the long-line passes, and
 // the generic shared-memory Stockham kernel otherwise (which uses the input
 // strides for its output too: it never sees the z-tiled layout)
 cudaError_t line_pass(PPLinePassArgs a, const DirTables& d, bool inverse, bool strided, bool in_cplx,
@@ -564,9 +571,7 @@ cudaError_t line_pass(PPLinePassArgs a, const DirTables& d, bool inverse, bool s
         a.o_plane_stride = a.plane_stride;
         a.o_tile_stride = a.tile_stride;
     }
-    int lpc = pp_lp2_lpc(d.n);
-    const bool mixed = lpc == 0 && pp_lpm_lpc(d.n) > 0;
-    if (mixed) lpc = pp_lpm_lpc(d.n);
+    const int lpc = pp_lp2_lpc(d.n);
     if (d.n1 > 0) {
         PPLongPlan lp{};
         lp.n1 = d.n1;
@@ -588,6 +593,13 @@ cudaError_t line_pass(PPLinePassArgs a, const DirTables& d, bool inverse, bool s
         }
         a.cs2 = d.csf.p;
         return pp_launch_long_line_pass(a, lp, inverse, strided, in_cplx, out_cplx, st, fp32);
+    }
+    // (the real families write complex points only as the solution P)
+    const PPMrPlan& mr = a.half ? d.mrh : d.mr;
+    if (lpc == 0 && mr.m > 0 && (d.kind == PP_KIND_FFT || !out_cplx || (inverse && !strided))) {
+        a.tw = fp32 ? d.twf.p : d.tw.p;
+        a.cs2 = fp32 ? d.csf.p : d.cs.p;
+        return pp_mr_line_pass(a, mr, inverse, strided, in_cplx, out_cplx, fp32, st);
     }
     if (fp32 && lpc == 0) {
         a.fft = d.fft;
@@ -613,9 +625,6 @@ cudaError_t line_pass(PPLinePassArgs a, const DirTables& d, bool inverse, bool s
         a.vec16 = runs_aligned16(a, strided, (in_cplx ? 2 : 1) * (fp32 ? sizeof(float) : sizeof(double)), dl);
         a.L = dl;
         a.tiles_per_plane = (a.nlines + dl - 1) / dl;
-        if (mixed)
-            return fp32 ? pp_launch_line_pass_mixed_f32(a, inverse, strided, st)
-                        : pp_launch_line_pass_mixed(a, inverse, strided, st);
         return fp32 ? pp_launch_line_pass_pow2<float, float, float>(a, inverse, strided, st)
                     : pp_launch_line_pass_pow2<double, double, double>(a, inverse, strided, st);
     }
@@ -672,25 +681,24 @@ void set_half_in(PPLinePassArgs& a, int ncol, long splane, int nx, long plane)
 // The forward y pass writes, and the inverse y pass reads, the spectrum as
 // contiguous z tiles (TS adjacent kx x all nz of one ky), so that the z solve
 // moves whole contiguous blocks; TS is the y pass's lines per tile.  Used
-// when the y pass is the register-resident kernel (power-of-two lengths,
-// 3 2^k and 5 2^k) with full tiles (nx a multiple of TS), the z solve is the
-// direct one and takes TS systems per CTA.
-int reg_lines(int n)
-{
-    const int lpc = pp_lp2_lpc(n);
-    return lpc ? lpc : pp_lpm_lpc(n);
-}
+// when the y pass takes strides of its own (every kernel but the generic one)
+// with full tiles (the columns a multiple of TS), the z solve is the direct one
+// and takes TS systems per CTA.
 // data lines per tile of the y pass (0: the generic kernel)
-int y_tile_lines(int n, bool cplx)
+int y_tile_lines(const DirTables& t)
 {
-    if (!cplx && pp_rh_lines(n, true)) return pp_rh_lines(n, true);
-    return cplx ? reg_lines(n) : 2 * reg_lines(n);
+    const bool cplx = t.kind == PP_KIND_FFT;
+    if (!cplx && pp_rh_lines(t.n, true)) return pp_rh_lines(t.n, true);
+    if (const int lpc = pp_lp2_lpc(t.n)) return cplx ? lpc : 2 * lpc;
+    return t.mr.m ? pp_mr_lines(t.n, t.kind, t.mr) : 0;
 }
 int z_tile_width(const pp_solver_s* h, bool s_cplx, int ncol)
 {
     if (h->opt.z_solver != PP_ZSOLVE_DIRECT || h->slab) return 0;
-    const int dl = y_tile_lines(h->ny, s_cplx);
-    if (dl < 2 || dl > 16 || ncol % dl != 0) return 0;
+    const int dl = y_tile_lines(h->ty);
+    // (rows of at least 64 bytes: on narrower ones the z solve's tiles are worth
+    // less than its own row segments, 1280 x 1280 x 64 periodic 0.85 and 0.49 ms)
+    if (dl * (s_cplx ? 16 : 8) < 64 || dl > 16 || ncol % dl != 0) return 0;
     if (h->tune.zsolve_tile != 0 && h->tune.zsolve_tile != dl) return 0;
     int ts = 0, threads = 0;
     pp_zsolve_config_p(h->nz, s_cplx, ncol, h->tune.zsolve_lanes, &ts, &threads, dl, h->ny);
@@ -705,8 +713,9 @@ int z_tile_width(const pp_solver_s* h, bool s_cplx, int ncol)
 // 0 when the path does not apply (the full complex spectrum is used).
 int half_spectrum_cols(const pp_solver_s* h)
 {
-    if (h->tx.kind != PP_KIND_FFT || h->rhs_complex || h->nx < 32 || reg_lines(h->nx) == 0) return 0;
-    int q = y_tile_lines(h->ny, h->ty.kind == PP_KIND_FFT);
+    if (h->tx.kind != PP_KIND_FFT || h->rhs_complex || h->nx < 32) return 0;
+    if (pp_lp2_lpc(h->nx) == 0 && h->tx.mrh.m == 0) return 0;
+    int q = y_tile_lines(h->ty);
     if (q == 0) q = 1;
     if (q > 16) q = 16;
     const int c = ((h->nx / 2 + 1 + q - 1) / q) * q;
@@ -1894,7 +1903,7 @@ int pp_autotune(pp_handle h, int reps, pp_tuning* chosen, double* best_ms)
         }
     }
     // generic transform kernel: lines per tile, only where it runs
-    const bool generic = reg_lines(h->nx) == 0 || reg_lines(h->ny) == 0;
+    const bool generic = (pp_lp2_lpc(h->nx) == 0 && h->tx.mr.m == 0) || (pp_lp2_lpc(h->ny) == 0 && h->ty.mr.m == 0);
     for (int L = 1; generic && L <= 32 && rc == PP_SUCCESS; L *= 2) {
         pp_tuning t = best;
         t.line_tile = L;
