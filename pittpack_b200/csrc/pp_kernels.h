@@ -258,7 +258,15 @@ bool pp_zsolve_ref_defined(int method, int nz, int zlo, int zhi);
 cudaError_t pp_launch_zsolve_ref(const PPZRefArgs& a, cudaStream_t st);
 
 struct pp_solver_s;
-// bytes of each of a handle's grid-sized buffers
+// columns a row of the spectrum may be padded by: up to a multiple of 16, or of
+// 8, where that is at most an eighth of it
+inline int pp_spare_cols(int nx)
+{
+    for (int q = 16; q >= 8; q /= 2)
+        if ((q - nx % q) % q <= nx / 8) return (q - nx % q) % q;
+    return 0;
+}
+// bytes of each of a handle's two spectrum buffers
 size_t pp_spectrum_bytes(int nx, int ny, int nz);
 // a handle (pp_destroy frees it) that works in its caller's memory: the two
 // spectrum buffers, and for the refined solve a quarter as much for the FP32

@@ -676,6 +676,16 @@ PP_D void mr_body(const PPLinePassArgs& a, const PPMrPlan& pl)
             put(0, 2 * i + 1, v.y);
         }
     };
+    // the padding columns of the spectrum's rows stay zero
+    if constexpr (!INV && !STR && K != K_HALF) {
+        for (int e = N + i0; e < (int)ols; e += G)
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+                if (d == 1 && !live2) continue;
+                if (a.out_cplx) dstc[d * ols + e] = mkc<C>(0, 0);
+                else dst[d * ols + e] = (Real)0;
+            }
+    }
     // DCT-II value pair of U = e^{-i t_k} V_k: X_k = 2 Re U, X_{N-k} = -2 Im U;
     // DST-II: output e = N-1-k with sign (-1)^e
     auto emit = [&](int d, int k, C V, C w, bool second) {
