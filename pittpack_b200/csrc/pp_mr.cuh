@@ -567,17 +567,7 @@ PP_D void mr_body(const PPLinePassArgs& a, const PPMrPlan& pl)
     } else {
         // inverse, even N: Z_k = A + i B, Z_{M-k} = conj(A - i B),
         // A = V_k + conj V_{M-k}, B = e^{2 pi i k / N} (V_k - conj V_{M-k})
-        staged<UH>(i0, H, G, [&](int k) {
-            if constexpr (K == K_HALF) {
-                const C p_ = srcc[k], q_ = srcc[M - k];
-                return Quad<Real, C>{p_.x, p_.y, q_.x, q_.y, C{}, __ldg(&tw[k])};
-            } else {
-                // X'_k, X'_{N-k}, X'_{M-k}, X'_{M+k}; X'_k = X_k, or (-1)^k X_{N-1-k} for DST-III
-                const int ea = dst2 ? N - 1 - k : k, eb = k == 0 ? ea : dst2 ? k - 1 : N - k;
-                const int ec = dst2 ? N - 1 - M + k : M - k, ed = dst2 ? N - 1 - M - k : M + k;
-                return Quad<Real, C>{X(ea), X(eb), X(ec), X(ed < 0 ? 0 : ed), __ldg(&cs[k]), __ldg(&tw[k])};
-            }
-        }, [&](int k, Quad<Real, C> x) {
+        auto use = [&](int k, Quad<Real, C> x) {
             C Vk, Vm;
             if constexpr (K == K_HALF) {
                 Vk = mkc<C>(x.a, k ? x.b : (Real)0);
@@ -608,7 +598,26 @@ PP_D void mr_body(const PPLinePassArgs& a, const PPMrPlan& pl)
             const C B = c_mul(mkc<C>(Vk.x - Vm.x, Vk.y + Vm.y), w);
             col[k * LP] = mkc<C>(A.x - B.y, A.y + B.x);
             if (k > 0 && 2 * k != M) col[(M - k) * LP] = mkc<C>(A.x + B.y, B.x - A.y);
-        });
+        };
+        if constexpr (K == K_HALF) {
+            if (a.in_cplx)
+                staged<UH>(i0, H, G, [&](int k) {
+                    const C p_ = srcc[k], q_ = srcc[M - k];
+                    return Quad<Real, C>{p_.x, p_.y, q_.x, q_.y, C{}, __ldg(&tw[k])};
+                }, use);
+            else  // the spectrum of a non-periodic y is real: the y transform drops the
+                  // imaginary part (src/signalProc.cpp:160-195)
+                staged<UH>(i0, H, G, [&](int k) {
+                    return Quad<Real, C>{src[k], (Real)0, src[M - k], (Real)0, C{}, __ldg(&tw[k])};
+                }, use);
+        } else {
+            staged<UH>(i0, H, G, [&](int k) {
+                // X'_k, X'_{N-k}, X'_{M-k}, X'_{M+k}; X'_k = X_k, or (-1)^k X_{N-1-k} for DST-III
+                const int ea = dst2 ? N - 1 - k : k, eb = k == 0 ? ea : dst2 ? k - 1 : N - k;
+                const int ec = dst2 ? N - 1 - M + k : M - k, ed = dst2 ? N - 1 - M - k : M + k;
+                return Quad<Real, C>{X(ea), X(eb), X(ec), X(ed < 0 ? 0 : ed), __ldg(&cs[k]), __ldg(&tw[k])};
+            }, use);
+        }
     }
     __syncthreads();
 

@@ -572,7 +572,18 @@ PP_D void rh_body(const PPLinePassArgs& a)
             const C* hi = reinterpret_cast<const C*>(src) + base + (M - t);
 #pragma unroll
             for (int j = 0; j < H; ++j) zk[j] = zm[j] = mkc<C>(0, 0);
-            if (live) {
+            if (live && !a.in_cplx) {
+                // the spectrum of a non-periodic y is real: the y transform drops the
+                // imaginary part (src/signalProc.cpp:160-195)
+                const Real* rl = src + base + t;
+                const Real* rh = src + base + (M - t);
+#pragma unroll
+                for (int j = 0; j < H; ++j) {
+                    zk[j].x = rl[T * j];
+                    zm[j].x = rh[-T * j];
+                }
+                if (t == 0) vh.x = rl[M / 2];
+            } else if (live) {
 #pragma unroll
                 for (int j = 0; j < H; ++j) {
                     zk[j] = lo[T * j];
