@@ -33,8 +33,16 @@
 //     on the system's last row;
 //   * eliminating each lane's first unknown leaves a P-row tridiagonal system
 //     in the lanes' last unknowns, solved by parallel cyclic reduction over
-//     warp shuffles (periodic systems through Sherman-Morrison); each lane
+//     warp shuffles (on the ring of lanes for periodic systems); each lane
 //     then recovers its interior rows;
+//   * every elimination carries a row by its off-diagonals and its sum, and
+//     forms the diagonal from them (Grassmann, Taksar and Heyman 1985; Alfa,
+//     Xue and Ye 2002): with lambda = -(2 + e) the matrix is a diagonally
+//     dominant M-matrix whose row sums (e inside) all steps only add up, so
+//     that nothing cancels where the lowest modes are nearly singular.  Error
+//     against the exact solution of a lowest mode's system, 2-norm, diagonals
+//     formed directly -> from the sums: 200 rows 5e-14 -> 3e-16, 300 rows
+//     1.3e-13 -> 3e-16, 512 rows 2.4e-13 -> 3e-16, whatever the number of lanes;
 //   * where a lane keeps 9 .. 34 rows (complex 9 .. 19) in registers, they form
 //     two blocks whose sweeps run side by side (two independent FP64
 //     recurrences per lane: the sweeps are bound by the latency of their
@@ -69,16 +77,6 @@ PP_D double zshfl(double v, int src, int w) { return __shfl_sync(0xffffffffu, v,
 PP_D double2 zshfl(double2 v, int src, int w)
 {
     return make_double2(__shfl_sync(0xffffffffu, v.x, src, w), __shfl_sync(0xffffffffu, v.y, src, w));
-}
-PP_D double zshfl_up(double v, int d, int w) { return __shfl_up_sync(0xffffffffu, v, d, w); }
-PP_D double2 zshfl_up(double2 v, int d, int w)
-{
-    return make_double2(__shfl_up_sync(0xffffffffu, v.x, d, w), __shfl_up_sync(0xffffffffu, v.y, d, w));
-}
-PP_D double zshfl_down(double v, int d, int w) { return __shfl_down_sync(0xffffffffu, v, d, w); }
-PP_D double2 zshfl_down(double2 v, int d, int w)
-{
-    return make_double2(__shfl_down_sync(0xffffffffu, v.x, d, w), __shfl_down_sync(0xffffffffu, v.y, d, w));
 }
 
 // asynchronous global -> shared copies (LDGSTS): no register staging, every
@@ -159,72 +157,79 @@ PP_D void zt_each(int TS, int lts, int nz, int ts, F f)
 
 // The reduced system of a lane group, one row per lane L in the lanes' last
 // unknowns l:  ra l_{L-1} + rb l_L + rc l_{L+1} = rd,  lane indices wrapping
-// (periodic z; otherwise ra = 0 on the first lane and rc = 0 on the last).
-// Solved by parallel cyclic reduction over warp shuffles, the periodic one
-// through Sherman-Morrison; returns l_L.
+// (periodic z; otherwise ra = 0 on the first lane and rc = 0 on the last),
+// given by its off-diagonals and its sum rs = ra + rb + rc.  Solved by parallel
+// cyclic reduction over warp shuffles on the ring of lanes: after log2 P steps
+// a row's neighbours on both sides are itself, and its sum is what is left (in
+// a chain the off-diagonals have become zero).  Returns l_L.
 template <typename T>
-PP_D T zsolve_reduced(double ra, double rb, double rc, T rd, int lane, int P, bool periodic)
+PP_D T zsolve_reduced(double ra, double rs, double rc, T rd, int lane, int P)
 {
-    if (P == 1)  // one row: its neighbours on both sides are itself
-        return zmul(1.0 / (ra + rb + rc), rd);
-    {
-        const double inv = 1.0 / rb;
+    const double inv0 = 1.0 / (P == 1 ? rs : rs - ra - rc);
+    rd = zmul(inv0, rd);
+    ra *= inv0;
+    rc *= inv0;
+    rs *= inv0;
+    for (int st = 1; st < P; st <<= 1) {
+        const int prv = (lane - st) & (P - 1), nxt = (lane + st) & (P - 1);
+        const double ap = zshfl(ra, prv, P), sp = zshfl(rs, prv, P);
+        const T dp = zshfl(rd, prv, P);
+        const double cn = zshfl(rc, nxt, P), sn = zshfl(rs, nxt, P);
+        const T dn = zshfl(rd, nxt, P);
+        // (the row's diagonal is 1; minus its off-diagonals times the neighbours' rows)
+        rs = rs - ra * sp - rc * sn;
+        rd = zsub(zsub(rd, zmul(ra, dp)), zmul(rc, dn));
+        ra = -ra * ap;
+        rc = -rc * cn;
+        const double inv = 1.0 / (2 * st == P ? rs : rs - ra - rc);
+        rd = zmul(inv, rd);
         ra *= inv;
         rc *= inv;
-        rd = zmul(inv, rd);
+        rs *= inv;
     }
-    double ru = 0.0, beta = 0.0;
-    const double gam = -1.0;
-    if (periodic) {
-        // the corners move into u v^T with u = (gam, 0, .., alpha),
-        // v = (1, 0, .., beta / gam): beta = a_0, alpha = c_{P-1}
-        beta = zshfl(ra, 0, P);
-        const double alpha = zshfl(rc, P - 1, P);
-        if (lane == 0) {
-            const double b0 = 1.0 - gam;
-            ra = 0.0;
-            rc /= b0;
-            rd = zmul(1.0 / b0, rd);
-            ru = gam / b0;
-        }
-        if (lane == P - 1) {
-            const double bl = 1.0 - alpha * beta / gam;
-            rc = 0.0;
-            ra /= bl;
-            rd = zmul(1.0 / bl, rd);
-            ru = alpha / bl;
-        }
+    return rd;
+}
+
+// The end rows of a block.  Every block has the same interior rows, so its two
+// end equations (zsolve_split) come from the pivot table at its last row k:
+//   E0: f + e0a l_prev + e0c l = ..   gamma_k, alpha_k, sum psi_k = 1 + gamma_k + alpha_k,
+//   E1: e1a f + l + e1c f_next = ..   alpha_k, gamma_k, the same sum.
+// A block that ends the system has no neighbour there, and its row is scaled:
+// by 1 / (psi_k - alpha_k) at a Neumann end (diagonal lambda + 1), by
+// 1 / (1 - gamma_k) at a Dirichlet one (lambda - 1).
+struct ZEnd {
+    double scale, c, sum;  // of the row: scale, coefficient across the block, sum
+};
+PP_D ZEnd zend(bool neumann, double g, double al, double psi)
+{
+    ZEnd e;
+    e.scale = 1.0 / (neumann ? psi - al : 1.0 - g);
+    e.c = al * e.scale;
+    e.sum = neumann ? psi * e.scale : 1.0 + e.c;
+    return e;
+}
+// coefficients of E0 (q: the factor of its right-hand side d_0 - (row 1's)),
+// modified on the system's first block; pin: row 0 is x_0 = d_0, or
+// x_0 + x_{nz-1} = d_0 for periodic z
+struct ZFirst {
+    double a, c, sum, q;
+};
+PP_D ZFirst zfirst(bool first, bool pin, bool periodic, bool neumann, double g, double al, double psi)
+{
+    ZFirst r = {g, al, psi, g};
+    if (first && pin) {
+        r.a = periodic ? 1.0 : 0.0;
+        r.c = 0.0;
+        r.sum = 1.0 + r.a;
+        r.q = 1.0;
+    } else if (first && !periodic) {
+        const ZEnd e = zend(neumann, g, al, psi);
+        r.a = 0.0;
+        r.c = e.c;
+        r.sum = e.sum;
+        r.q = g * e.scale;
     }
-    for (int st = 1; st < P; st <<= 1) {
-        const bool hp = lane >= st, hn = lane + st < P;
-        double ap = zshfl_up(ra, st, P), cp = zshfl_up(rc, st, P);
-        T dp = zshfl_up(rd, st, P);
-        double an = zshfl_down(ra, st, P), cn = zshfl_down(rc, st, P);
-        T dnx = zshfl_down(rd, st, P);
-        if (!hp) {
-            ap = cp = 0.0;
-            dp = zzero<T>();
-        }
-        if (!hn) {
-            an = cn = 0.0;
-            dnx = zzero<T>();
-        }
-        const double inv = 1.0 / (1.0 - ra * cp - rc * an);
-        if (periodic) {
-            const double up = zshfl_up(ru, st, P), un = zshfl_down(ru, st, P);
-            ru = (ru - ra * (hp ? up : 0.0) - rc * (hn ? un : 0.0)) * inv;
-        }
-        rd = zmul(inv, zsub(zsub(rd, zmul(ra, dp)), zmul(rc, dnx)));
-        ra = -ra * ap * inv;
-        rc = -rc * cn * inv;
-    }
-    if (!periodic) return rd;
-    // fact = (y_0 + (beta/gam) y_{P-1}) / (1 + z_0 + (beta/gam) z_{P-1})
-    const double bg = beta / gam;
-    const T y0 = zshfl(rd, 0, P), yl = zshfl(rd, P - 1, P);
-    const double z0 = zshfl(ru, 0, P), zl = zshfl(ru, P - 1, P);
-    const T fact = zmul(1.0 / (1.0 + z0 + bg * zl), zadd(y0, zmul(bg, yl)));
-    return zsub(rd, zmul(ru, fact));
+    return r;
 }
 
 // The partition solve of one system by its lane group with each lane's MT
@@ -240,72 +245,36 @@ PP_D T zsolve_reduced(double ra, double rb, double rc, T rd, int lane, int P, bo
 // eliminating l_A (its neighbours l_B of the previous lane and of this one)
 // leaves one row per lane in the l_B's, solved by zsolve_reduced; l_A, both
 // f's and the blocks' interior rows follow.  tab holds the interior pivots of
-// a block of H rows (gamma_i, alpha_i, i < H); d0 is row 0's right-hand side
-// (after the periodic zero-mode averaging); row 0 of the system is the first
-// row of A on lane 0 and row nz - 1 the last row of B on lane P - 1.
+// a block of H rows (gamma_i, alpha_i, i < H), psiA and psiB the sums of the
+// blocks' end rows; d0 is row 0's right-hand side (after the periodic
+// zero-mode averaging); row 0 of the system is the first row of A on lane 0
+// and row nz - 1 the last row of B on lane P - 1.
 // UNEV: a lane has M = MT, MT - 1 or MT - 2 rows; block B is the shorter one
 // (HB = M - H rows), the branches on it are confined to its last three rows.
 template <int MT, bool UNEV, typename T>
-PP_D void zsolve_split(T (&xr)[MT], const double2* tab, T d0, int M, bool live, bool clear, int lane, int P,
-                       bool periodic, double lam, double A0, double B0, double C0, double AN, double BN,
-                       double CN)
+PP_D void zsolve_split(T (&xr)[MT], const double2* tab, double psiA, double psiB, T d0, int M, bool live, bool clear,
+                       int lane, int P, bool periodic, bool pin, bool nlo, bool nhi)
 {
     constexpr int H = MT / 2;
     static_assert(H >= (UNEV ? 5 : 4), "blocks of at least four rows, three in the shorter one");
     const int HB = UNEV ? M - H : H;
     const double* tg = reinterpret_cast<const double*>(tab);  // gamma_i = tg[2i], alpha_i = tg[2i+1]
-    const bool last = lane == P - 1;
     // ---- forward sweeps of A and B ----------------------------------------------------
     T dA = zzero<T>(), dB = zzero<T>();
-    double gA = 0.0, gB = 0.0, aA = 0.0, aB = 0.0;
     if (live) {
-        bool lastB = false;
 #pragma unroll
         for (int i = 1; i < H; ++i) {
             const double ga = tg[2 * i];
-            const T nA = (i == 1) ? zmul(ga, xr[i]) : zmul(ga, zsub(xr[i], dA));
-            T nB = zzero<T>();
-            // (rows above H - 4 may be B's last one, or past it)
-            const bool ends = UNEV && i > H - 4 ? i == HB - 1 : i == H - 1;
-            const bool past = UNEV && i > H - 3 && i > HB - 1;
-            if (past) {
-                xr[i] = nA;
-                dA = nA;
-                gA = ga;
-                continue;
-            }
-            if (ends && last) {
-                // the system's last row closes B on the last lane
-                const double p = 1.0 / (BN - AN * gB);
-                aB = -AN * tg[2 * (i - 1) + 1] * p;
-                gB = CN * p;
-                nB = zmul(p, zsub(xr[H + i], zmul(AN, dB)));
-                lastB = true;
-            } else {
-                nB = (i == 1) ? zmul(ga, xr[H + i]) : zmul(ga, zsub(xr[H + i], dB));
-                gB = ga;
-            }
-            xr[i] = nA;
-            xr[H + i] = nB;
-            dA = nA;
-            dB = nB;
-            gA = ga;
+            dA = (i == 1) ? zmul(ga, xr[i]) : zmul(ga, zsub(xr[i], dA));
+            xr[i] = dA;
+            if (UNEV && i > H - 3 && i > HB - 1) continue;  // past B's last row
+            dB = (i == 1) ? zmul(ga, xr[H + i]) : zmul(ga, zsub(xr[H + i], dB));
+            xr[H + i] = dB;
         }
-        aA = tg[2 * (H - 1) + 1];
-        if (!lastB) aB = UNEV ? tg[2 * (HB - 1) + 1] : aA;
     }
     // ---- backward sweeps: row 1 of a block in terms of its first and last unknowns
-    double br = 0.0, cr = 0.0, brB = 0.0, crB = 0.0;
     T rA = zzero<T>(), rB = zzero<T>();
     if (live) {
-        const double2 t2 = tab[H - 2];
-        br = brB = t2.x;
-        cr = crB = t2.y;
-        if (UNEV) {
-            const double2 u2 = tab[HB - 2];
-            brB = u2.x;
-            crB = u2.y;
-        }
         rA = xr[H - 2];
         rB = xr[MT - 2];
 #pragma unroll
@@ -317,37 +286,41 @@ PP_D void zsolve_split(T (&xr)[MT], const double2* tab, T d0, int M, bool live, 
             else rB = zsub(xr[H + i], zmul(g, rB));
         }
     }
-    // ---- E0 of both blocks (A's first row is the system's row 0 on lane 0) -----------
-    const bool first = lane == 0;
-    const double a0 = first ? A0 : 1.0, b0 = first ? B0 : lam, c0 = first ? C0 : 1.0;
-    const double qA = 1.0 / (b0 - c0 * br);
-    const double e0aA = a0 * qA, e0cA = -c0 * cr * qA;
-    const T e0dA = zmul(qA, zsub(d0, zmul(c0, rA)));
-    const double qB = 1.0 / (lam - brB);
-    const double e0aB = qB, e0cB = -crB * qB;
-    const T e0dB = zmul(qB, zsub(live ? xr[H] : zzero<T>(), rB));
-    // ---- rows of the blocks' last unknowns --------------------------------------------
+    // ---- E0 and E1 of both blocks -------------------------------------------------------
+    const double2 tA = tab[H - 1], tB = UNEV ? tab[HB - 1] : tA;
+    const ZFirst fa = zfirst(lane == 0, pin, periodic, nlo, tA.x, tA.y, psiA);
+    const T e0dA = zmul(fa.q, zsub(d0, lane == 0 && pin ? zzero<T>() : rA));
+    const T e0dB = zmul(tB.x, zsub(live ? xr[H] : zzero<T>(), rB));
+    double e1aB = tB.y, e1cB = tB.x, e1sB = psiB;
+    if (lane == P - 1 && !periodic) {
+        const ZEnd e = zend(nhi, tB.x, tB.y, psiB);
+        e1aB = e.c;
+        e1cB = 0.0;
+        e1sB = e.sum;
+        dB = zmul(e.scale, dB);
+    }
+    // ---- rows of the blocks' last unknowns (off-diagonals and sums) ---------------------
     // l_A:  raA l_B(prev lane) + rbA l_A + rcA l_B = rdA
-    const double raA = -aA * e0aA, rbA = 1.0 - aA * e0cA - gA * e0aB, rcA = -gA * e0cB;
-    const T rdA = zsub(zsub(dA, zmul(aA, e0dA)), zmul(gA, e0dB));
+    const double raA = -tA.y * fa.a, rcA = -tA.x * tB.y, rsA = psiA - tA.y * fa.sum - tA.x * psiB;
+    const T rdA = zsub(zsub(dA, zmul(tA.y, e0dA)), zmul(tA.x, e0dB));
     // l_B:  raB l_A + rbB l_B + rcB l_A(next lane) = rdB
     const int nxt = (lane + 1) & (P - 1);
-    const double na0 = zshfl(e0aA, nxt, P), nc0 = zshfl(e0cA, nxt, P);
+    const double nc0 = zshfl(fa.c, nxt, P), ns0 = zshfl(fa.sum, nxt, P);
     const T nd0 = zshfl(e0dA, nxt, P);
-    const double raB = -aB * e0aB, rbB = 1.0 - aB * e0cB - gB * na0, rcB = -gB * nc0;
-    const T rdB = zsub(zsub(dB, zmul(aB, e0dB)), zmul(gB, nd0));
+    const double raB = -e1aB * tB.x, rcB = -e1cB * nc0, rsB = e1sB - e1aB * psiB - e1cB * ns0;
+    const T rdB = zsub(zsub(dB, zmul(e1aB, e0dB)), zmul(e1cB, nd0));
     // l_A = pd - pa l_B(prev lane) - pc l_B, substituted into the l_B rows
-    const double iA = 1.0 / rbA;
-    const double pa = raA * iA, pc = rcA * iA;
+    const double iA = 1.0 / (rsA - raA - rcA);
+    const double pa = raA * iA, pc = rcA * iA, ps = rsA * iA;
     const T pd = zmul(iA, rdA);
-    const double npa = zshfl(pa, nxt, P), npc = zshfl(pc, nxt, P);
+    const double npc = zshfl(pc, nxt, P), nps = zshfl(ps, nxt, P);
     const T npd = zshfl(pd, nxt, P);
-    const T lB = zsolve_reduced(-raB * pa, rbB - raB * pc - rcB * npa, -rcB * npc,
-                                zsub(zsub(rdB, zmul(raB, pd)), zmul(rcB, npd)), lane, P, periodic);
+    const T lB = zsolve_reduced(-raB * pa, rsB - raB * ps - rcB * nps, -rcB * npc,
+                                zsub(zsub(rdB, zmul(raB, pd)), zmul(rcB, npd)), lane, P);
     const T lBp = zshfl(lB, (lane + P - 1) & (P - 1), P);
     const T lA = zsub(zsub(pd, zmul(pa, lBp)), zmul(pc, lB));
-    const T fA = zsub(zsub(e0dA, zmul(e0aA, lBp)), zmul(e0cA, lA));
-    const T fB = zsub(zsub(e0dB, zmul(e0aB, lA)), zmul(e0cB, lB));
+    const T fA = zsub(zsub(e0dA, zmul(fa.a, lBp)), zmul(fa.c, lA));
+    const T fB = zsub(zsub(e0dB, zmul(tB.x, lA)), zmul(tB.y, lB));
     // ---- recover both blocks' rows ------------------------------------------------------
     if (!live) return;
     if (clear) {
@@ -402,7 +375,7 @@ PP_HD ZLayout zlayout(int TS, int nz, int P, bool cplx, int nthreads, bool g32 =
     const size_t chunks = (size_t)P * (((size_t)(nz + P - 1) / P) * TS * e + 16);
     if (chunks > L.tab_off) L.tab_off = chunks;
     L.tab_off = (L.tab_off + 15) & ~(size_t)15;
-    // scratch of the pivot-table build: the b_i recurrence of every system
+    // scratch of the pivot-table build: the u_i recurrence of every system
     L.red_off = L.tab_off + (size_t)TS * L.mmax * 16;
     L.bytes = L.red_off + (size_t)TS * L.mmax * 8;
     L.stg_off = (L.bytes + 15) & ~(size_t)15;
@@ -520,57 +493,71 @@ PP_D void zsolve_body(PPZArgs a)
             });
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
-    // interior pivots of a block, depending only on lambda: with b_0 = 1,
-    // b_1 = lambda, b_i = lambda b_{i-1} - b_{i-2} (Chebyshev U_i(lambda/2)),
-    //   gamma_i = b_{i-1} / b_i,  alpha_i = (-1)^{i-1} / b_i,
-    // the same numbers as the Thomas recurrence gamma_i = 1 / (lambda - gamma_{i-1}).
-    // One thread per system; the divisions are independent.  |b_i| grows like
+    // interior pivots of a block, depending only on lambda = -(2 + e): with
+    // u_0 = 1, u_1 = 2 + e, u_i = (2 + e) u_{i-1} - u_{i-2} (Chebyshev U_i(1 + e/2)),
+    //   gamma_i = -u_{i-1} / u_i,  alpha_i = -1 / u_i,
+    // the same numbers as the Thomas recurrence gamma_i = 1 / (lambda - gamma_{i-1}),
+    // and the sums psi_i = 1 + gamma_i + alpha_i = w_i / u_i, w_i = e (u_0 + .. + u_{i-1}),
+    // of the end rows.  By the differences v_i = u_i - u_{i-1} = v_{i-1} + e u_{i-1} = 1 + w_i
+    // all are sums of positive terms: full relative accuracy for any e >= 0.
+    // One thread per system; the divisions are independent.  u_i grows like
     // |lambda|^i, so where mm log2|lambda| could leave the double range the
     // division recurrence is used instead.
-    // Phase 1, one thread per system: b_i by the recurrence (FMAs only) into
-    // the scratch bytes, or -- where |b_i| could overflow -- the division
-    // recurrence straight into the table, marked by b_0 = 0.
+    // Phase 1, one thread per system: u_i by the recurrence (FMAs only) into
+    // the scratch bytes, or -- where u_i could overflow -- the division
+    // recurrence straight into the table, marked by u_0 = 0.
     double* bsc = reinterpret_cast<double*>(zsm_raw + Lz.red_off);
     const int mm = Lz.mmax;
-    const int mcount = SPLIT ? MT / 2 : mm;  // entries built (split blocks: MT / 2 rows)
+    const int mcount = SPLIT ? MT / 2 : mm - 1;  // rows of the longest block: entries 1 .. mcount - 1
+    // psi of the last row of the longest block, of one a row shorter (both in the
+    // table's unused entry 0) and of one two rows shorter (past the scratch's u_i)
+    auto psi_of = [&](int s, int j) -> double& {
+        double* t0 = reinterpret_cast<double*>(zsm_raw + Lz.tab_off) + 2 * (size_t)s * mm;
+        return j < 2 ? t0[j] : bsc[(size_t)s * mm + mm - 1];
+    };
     for (int s = threadIdx.x; s < ts; s += blockDim.x) {
         const double lam = (-2.0 + a.ax[kx0 + s] * a.Cx) + a.ay[ky] * a.Cy;
-        double* b = bsc + (size_t)s * mm;
+        const double e = -(lam + 2.0);
+        double* u = bsc + (size_t)s * mm;
         if ((double)mcount * log2(fabs(lam) + 1.0) < 900.0) {
-            double bm = 1.0, bc = lam;
-            b[0] = 1.0;
+            double uc = 1.0, v = 1.0, w = 0.0;
+            u[0] = 1.0;
             for (int i = 1; i < mcount; ++i) {
-                b[i] = bc;
-                const double bn = lam * bc - bm;
-                bm = bc;
-                bc = bn;
+                w += e * uc;
+                v += e * uc;
+                uc += v;
+                u[i] = uc;
+                if (i >= mcount - 3) psi_of(s, mcount - 1 - i) = w;  // (divided by u_i in phase 2)
             }
         } else {
+            // q_i = 1 + t_i = 2 + e - 1 / q_{i-1}, t_i = e + t_{i-1} / q_{i-1};
+            // gamma_i = -1 / q_i, alpha_i = alpha_{i-1} / q_i, psi_i = (e + psi_{i-1}) / q_i
             double2* tb = reinterpret_cast<double2*>(zsm_raw + Lz.tab_off) + (size_t)s * mm;
-            double gp = 0.0, ap = 0.0;
+            double t = 1.0 + e, al = -1.0, psi = 0.0;
             for (int i = 1; i < mcount; ++i) {
-                const double p = (i == 1) ? 1.0 / lam : 1.0 / (lam - gp);
-                const double al = (i == 1) ? p : -ap * p;
-                tb[i] = make_double2(p, al);
-                gp = p;
-                ap = al;
+                const double p = 1.0 / (1.0 + t);
+                al *= p;
+                psi = (e + psi) * p;
+                tb[i] = make_double2(-p, al);
+                if (i >= mcount - 3) psi_of(s, mcount - 1 - i) = psi;
+                t = e + t * p;
             }
-            b[0] = 0.0;
+            u[0] = 0.0;
         }
     }
     __syncthreads();
-    // Phase 2, every thread: gamma_i = b_{i-1} / b_i, alpha_i = (-1)^{i-1} / b_i,
-    // one reciprocal per entry, the entries of all systems spread over the CTA
+    // Phase 2, every thread: gamma_i = -u_{i-1} / u_i, alpha_i = -1 / u_i, one
+    // reciprocal per entry, the entries of all systems spread over the CTA
     {
         // blockDim.x / TS threads per system (both powers of two)
         const int ltp = __ffs(blockDim.x) - 1 - lts;
         const int s = threadIdx.x >> ltp;
-        const double* b = bsc + (size_t)s * mm;
-        if (s < ts && b[0] != 0.0)
+        const double* u = bsc + (size_t)s * mm;
+        if (s < ts && u[0] != 0.0)
             for (int i = (threadIdx.x & ((1 << ltp) - 1)) + 1; i < mcount; i += 1 << ltp) {
-                const double inv = 1.0 / b[i];
-                reinterpret_cast<double2*>(zsm_raw + Lz.tab_off)[(size_t)s * mm + i] =
-                    make_double2(b[i - 1] * inv, (i & 1) ? inv : -inv);
+                const double inv = -1.0 / u[i];
+                reinterpret_cast<double2*>(zsm_raw + Lz.tab_off)[(size_t)s * mm + i] = make_double2(u[i - 1] * inv, inv);
+                if (i >= mcount - 3) psi_of(s, mcount - 1 - i) *= -inv;
             }
     }
     cp_async_wait_all();
@@ -646,22 +633,8 @@ PP_D void zsolve_body(PPZArgs a)
             else return col[zpos(s0 + i)];
         };
 
-        double A0, B0, C0, AN, BN, CN;
-        if (periodic) {
-            A0 = 1.0;
-            B0 = pin ? 1.0 : lam;
-            C0 = pin ? 0.0 : 1.0;
-            AN = 1.0;
-            BN = lam;
-            CN = 1.0;
-        } else {
-            A0 = 0.0;
-            B0 = pin ? 1.0 : (a.zlo == PP_Z_NEUMANN ? lam + 1. : lam - 1.);
-            C0 = pin ? 0.0 : 1.0;
-            AN = 1.0;
-            BN = a.zhi == PP_Z_NEUMANN ? lam + 1.0 : lam - 1.;
-            CN = 0.0;
-        }
+        // a Neumann first / last row, else a Dirichlet one
+        const bool nlo = a.zlo == PP_Z_NEUMANN, nhi = a.zhi == PP_Z_NEUMANN;
 
         if constexpr (SPLIT) {
             T d0 = zzero<T>();
@@ -673,21 +646,13 @@ PP_D void zsolve_body(PPZArgs a)
                     d0 = zmul(0.5, zadd(d0, last));
                 }
             }
-            zsolve_split<MT, CAP>(xr, tab, d0, M, live, zero && a.skip_zero, lane, P, periodic, lam, A0, B0, C0, AN, BN, CN);
+            zsolve_split<MT, CAP>(xr, tab, psi_of(live ? s : 0, 0), psi_of(live ? s : 0, CAP ? MT - M : 0), d0, M, live,
+                                  zero && a.skip_zero, lane, P, periodic, pin, nlo, nhi);
         } else {
             // ---- forward sweep of the lane's block -------------------------------------
             // row i (i >= 1) becomes alpha_i x_0 + x_i + gamma_i x_{i+1} = delta_i; delta
             // overwrites the RHS in the tile (only this lane touches these rows)
-            double rA0 = 1.0, rB0 = lam, rC0 = 1.0;
-            if (s0 == 0) {
-                rA0 = A0;
-                rB0 = B0;
-                rC0 = C0;
-            }
             T rD0 = zzero<T>(), dprev = zzero<T>();
-            // alpha of the block's last row: the table's, or the system's last row
-            double aprev = 0.0, gprev = 0.0;
-            bool last_special = false;
             const double* tg = reinterpret_cast<const double*>(tab);  // gamma_i = tg[2i], alpha_i = tg[2i+1]
             if (live) {
                 rD0 = X(0);
@@ -702,54 +667,18 @@ PP_D void zsolve_body(PPZArgs a)
 #pragma unroll
                 for (int i = 1; i < (MT > 0 ? MT : M); ++i) {
                     if (CAP && i >= M) break;
-                    const int gk = s0 + i;
                     const T D = X(i);
-                    double ga;
-                    T dn;
-                    // with MT rows per lane only the last unrolled row can be the
-                    // system's last row: for real spectra the test is resolved at
-                    // compile time elsewhere (for complex ones the register cost of
-                    // the specialised code outweighs it).  Interior rows need gamma
-                    // only; alpha matters for the block's last row alone.
-                    if (!((MT == 0 || CAP || CPLX || i == MT - 1) && gk == nz - 1)) {
-                        ga = tg[2 * i];
-                        dn = (i == 1) ? zmul(ga, D) : zmul(ga, zsub(D, dprev));
-                    } else if (i == 1) {
-                        const double inv = 1.0 / BN;
-                        aprev = AN * inv;
-                        ga = CN * inv;
-                        dn = zmul(inv, D);
-                        last_special = true;
-                    } else {
-                        const double p = 1.0 / (BN - AN * gprev);
-                        aprev = -AN * tg[2 * (i - 1) + 1] * p;
-                        ga = CN * p;
-                        dn = zmul(p, zsub(D, zmul(AN, dprev)));
-                        last_special = true;
-                    }
-                    X(i) = dn;
-                    gprev = ga;
-                    dprev = dn;
+                    dprev = (i == 1) ? zmul(tg[2 * i], D) : zmul(tg[2 * i], zsub(D, dprev));
+                    X(i) = dprev;
                 }
-                if (!last_special) aprev = tg[2 * (M - 1) + 1];
             }
-            // (alpha, gamma, delta) of the block's last row: the reduced row E1
-            const double e1a = aprev, e1c = gprev;
-            const T e1d = dprev;
             __syncwarp(full);
 
             // ---- backward sweep: row 1 in terms of x_0 and x_{M-1} ------------------------
-            // x_1 = dr - br x_0 - cr x_{M-1}.  The spikes are entries of the inverse
-            // of the block's interior matrix tridiag(1, lambda, 1) of order n = M-2:
-            // br = [T^-1]_11 = b_{n-1} / b_n = gamma_n and cr = [T^-1]_1n =
-            // (-1)^{n+1} / b_n = alpha_n, both in the table; only dr is swept.
-            double br = 0, cr = 0;
+            // x_1 = dr - gamma_{M-2} x_0 - alpha_{M-2} x_{M-1} (the spikes are entries of
+            // the inverse of the block's interior matrix); only dr is swept.
             T dr = zzero<T>();
             if (live && M >= 3) {
-                const double2 t2 = tab[M - 2];
-                br = t2.x;
-                cr = t2.y;
-                const double* tg = reinterpret_cast<const double*>(tab);
                 if constexpr (CAP) {
                     // registers indexed statically: rows above M - 2 are skipped
 #pragma unroll
@@ -763,40 +692,39 @@ PP_D void zsolve_body(PPZArgs a)
                     for (int i = M - 3; i >= 1; --i) dr = zsub(X(i), zmul(tg[2 * i], dr));
                 }
             }
-            double e0a, e0c;
-            T e0d;
-            if (M == 2) {
-                const double inv = 1.0 / rB0;
-                e0a = rA0 * inv;
-                e0c = rC0 * inv;
-                e0d = zmul(inv, rD0);
-            } else {
-                const double q = 1.0 / (rB0 - rC0 * br);
-                e0a = rA0 * q;
-                e0c = -rC0 * cr * q;
-                e0d = zmul(q, zsub(rD0, zmul(rC0, dr)));
+            // ---- E0 and E1 ----------------------------------------------------------------
+            // E0: f_L + e0a l_{L-1} + e0c l_L = e0d,  E1: e1a f_L + l_L + e1c f_{L+1} = e1d
+            // in the lane's first (f) and last (l) unknowns
+            const double2 tk = tab[M - 1];
+            const double psi = psi_of(live ? s : 0, EXACT ? 0 : mcount - M);
+            const ZFirst fa = zfirst(lane == 0, pin, periodic, nlo, tk.x, tk.y, psi);
+            const double e0a = fa.a, e0c = fa.c;
+            const T e0d = zmul(fa.q, zsub(rD0, lane == 0 && pin ? zzero<T>() : dr));
+            double e1a = tk.y, e1c = tk.x, e1s = psi;
+            T e1d = dprev;
+            if (lane == P - 1 && !periodic) {
+                const ZEnd e = zend(nhi, tk.x, tk.y, psi);
+                e1a = e.c;
+                e1c = 0.0;
+                e1s = e.sum;
+                e1d = zmul(e.scale, e1d);
             }
 
             // ---- reduced system ---------------------------------------------------------------
-            // lane L's rows E0: f_L + e0a l_{L-1} + e0c l_L = e0d and
-            //                E1: e1a f_L + l_L + e1c f_{L+1} = e1d
-            // in its first (f) and last (l) unknowns.  Eliminating every f_L with E0
-            // leaves a tridiagonal system in l alone, one row per lane (the Schur
-            // complement, diagonally dominant with the original):
-            //   -e1a e0a l_{L-1} + (1 - e1a e0c - e1c e0a') l_L - e1c e0c' l_{L+1}
-            //       = e1d - e1a e0d - e1c e0d'          (' : lane L+1)
+            // Eliminating every f_L with E0 leaves a tridiagonal system in l alone, one
+            // row per lane (the Schur complement, an M-matrix with the original):
+            //   -e1a e0a l_{L-1} + .. l_L - e1c e0c' l_{L+1} = e1d - e1a e0d - e1c e0d'
+            // of sum e1s - e1a e0s - e1c e0s'   (' : lane L+1)
             // The lane indices wrap (periodic z); without it e0a = 0 on the first lane
             // and e1c = 0 on the last, so the wrapped values carry no weight.  It is
-            // solved by parallel cyclic reduction over warp shuffles, the periodic one
-            // through Sherman-Morrison, and f_L follows from E0.
+            // solved by parallel cyclic reduction over warp shuffles, and f_L follows
+            // from E0.
             const int nxt = (lane + 1) & (P - 1);
-            const double na0 = zshfl(e0a, nxt, P), nc0 = zshfl(e0c, nxt, P);
+            const double nc0 = zshfl(e0c, nxt, P), ns0 = zshfl(fa.sum, nxt, P);
             const T nd0 = zshfl(e0d, nxt, P);
-            double ra = -e1a * e0a;
-            const double rb = 1.0 - e1a * e0c - e1c * na0;
-            double rc = -e1c * nc0;
-            T rd = zsub(zsub(e1d, zmul(e1a, e0d)), zmul(e1c, nd0));
-            const T xl = zsolve_reduced(ra, rb, rc, rd, lane, P, periodic);
+            const double ra = -e1a * e0a, rc = -e1c * nc0, rs = e1s - e1a * fa.sum - e1c * ns0;
+            const T rd = zsub(zsub(e1d, zmul(e1a, e0d)), zmul(e1c, nd0));
+            const T xl = zsolve_reduced(ra, rs, rc, rd, lane, P);
             const T xlp = zshfl(xl, (lane + P - 1) & (P - 1), P);
             const T xf = zsub(zsub(e0d, zmul(e0a, xlp)), zmul(e0c, xl));
             // ---- recover the block's rows ---------------------------------------------------
