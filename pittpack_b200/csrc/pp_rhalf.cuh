@@ -322,7 +322,7 @@ PP_D void put_runs(const PPLinePassArgs& a, long off, int stride, int plane, con
     }
     if (a.out_cplx) {
         C* d = reinterpret_cast<C*>(a.dst) + off;
-        if constexpr (sizeof(Real) == 8) {
+        if constexpr (sizeof(Real) == 8 && CNT % 2 == 0) {  // (vec_out: pairs of points start on 32 bytes)
             if (a.vec_out) {
 #pragma unroll
                 for (int q = 0; q < Q; ++q)
