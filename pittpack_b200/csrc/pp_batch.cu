@@ -88,7 +88,8 @@ int build_handles(pp_batch_s* b, const pp_batch_item* items, int n, const pp_opt
         size_t bytes = 0;
         for (int i = k; i < n; i += branches) {
             const pp_batch_item& it = items[i];
-            if (it.nx > 0 && it.ny > 0 && it.nz > 0) bytes = std::max(bytes, pp_spectrum_bytes(it.nx, it.ny, it.nz));
+            if (it.nx > 0 && it.ny > 0 && it.nz > 0)
+                bytes = std::max(bytes, pp_spectrum_bytes(it.nx, it.ny, it.nz, it.bc[2] == 'P'));
         }
         const size_t want[3] = {bytes, bytes, refined ? bytes / 4 : 0};
         for (int q = 0; q < 3; ++q)
@@ -104,7 +105,8 @@ int build_handles(pp_batch_s* b, const pp_batch_item* items, int n, const pp_opt
         const pp_batch_item& it = items[i];
         pp_handle h = nullptr;
         void* const* w = b->work[i % branches].p;
-        if ((rc = pp_create_lent(it.nx, it.ny, it.nz, w[0], w[1], w[2], &h)) != PP_SUCCESS) break;
+        const size_t bytes = pp_spectrum_bytes(it.nx, it.ny, it.nz, it.bc[2] == 'P');
+        if ((rc = pp_create_lent(it.nx, it.ny, it.nz, w[0], w[1], bytes, w[2], &h)) != PP_SUCCESS) break;
         b->handles.push_back(h);
         if ((rc = pp_set_box(h, it.box)) != PP_SUCCESS) break;
         if ((rc = pp_assign_boundary(h, it.bc)) != PP_SUCCESS) break;

@@ -266,11 +266,17 @@ inline int pp_spare_cols(int nx)
         if ((q - nx % q) % q <= nx / 8) return (q - nx % q) % q;
     return 0;
 }
-// bytes of each of a handle's two spectrum buffers
-size_t pp_spectrum_bytes(int nx, int ny, int nz);
+// bytes of each of a handle's two spectrum buffers: the complex points of the
+// grid, which hold the padding columns of real spectra too, and where y is
+// periodic (its spectrum may be complex) the padding columns beside them
+size_t pp_spectrum_bytes(int nx, int ny, int nz, bool y_periodic);
+// whether a handle may pad complex spectra (default: yes): pp_assign_boundary
+// then enlarges the spectrum buffers where the memory is there
+void pp_allow_padding(pp_solver_s* h, bool allow);
 // a handle (pp_destroy frees it) that works in its caller's memory: the two
-// spectrum buffers, and for the refined solve a quarter as much for the FP32
-// residual (null otherwise).  The caller binds the right-hand side and the
-// solution (pp_bind_device_buffers) before a solve, keeps the memory longer than
-// the handle, and runs handles that share it one after the other.
-int pp_create_lent(int nx, int ny, int nz, void* spec_a, void* spec_b, void* work, pp_solver_s** out);
+// spectrum buffers of 'bytes' (pp_spectrum_bytes), and for the refined solve a
+// quarter as much for the FP32 residual (null otherwise).  The caller binds the
+// right-hand side and the solution (pp_bind_device_buffers) before a solve,
+// keeps the memory longer than the handle, and runs handles that share it one
+// after the other.
+int pp_create_lent(int nx, int ny, int nz, void* spec_a, void* spec_b, size_t bytes, void* work, pp_solver_s** out);

@@ -239,6 +239,7 @@ struct pp_solver_s {
     cudaStream_t stream = 0;
     DirTables tx, ty;
     DevBuf rhs, bufA, bufB, out;
+    bool may_pad = true;  // complex spectra may be padded (pp_allow_padding)
     // caller-owned device buffers bound by pp_bind_device_buffers (zero copy):
     // the solve reads the RHS from ext_rhs and writes P to ext_out
     const double* ext_rhs = nullptr;
@@ -731,14 +732,41 @@ int half_spectrum_cols(const pp_solver_s* h)
 // transform passes as before).  The padding columns are zeros throughout.  Only where the x pass
 // writes rows of their own stride (the planned kernel: every other one's nx is
 // a multiple already, or has no strides of its own), not for slabs or the
-// alternate z solvers.
-int spectrum_cols(const pp_solver_s* h, int half)
+// alternate z solvers, and only as far as the spectrum buffers reach.
+int padded_cols(const pp_solver_s* h)
 {
-    if (half) return half;
     const int q = y_tile_lines(h->ty);
     if (h->slab || h->opt.z_solver != PP_ZSOLVE_DIRECT || q == 0 || pp_lp2_lpc(h->nx) || h->tx.mr.m == 0) return h->nx;
     const int c = (h->nx + q - 1) / q * q;
     return c <= h->nx + pp_spare_cols(h->nx) ? c : h->nx;
+}
+size_t padded_bytes(const pp_solver_s* h)
+{
+    const bool cplx = h->tx.kind == PP_KIND_FFT || h->ty.kind == PP_KIND_FFT;
+    return (cplx ? 2 : 1) * sizeof(double) * (size_t)padded_cols(h) * h->ny * h->nz;
+}
+int spectrum_cols(const pp_solver_s* h, int half)
+{
+    if (half) return half;
+    return padded_bytes(h) <= std::min(h->bufA.bytes, h->bufB.bytes) ? padded_cols(h) : h->nx;
+}
+
+// room for the padding columns of a complex spectrum, both buffers or neither:
+// without it the rows stay nx columns wide
+void grow_spectra(pp_solver_s* h)
+{
+    const size_t need = padded_bytes(h);
+    if (!h->may_pad || h->bufA.lent || h->ty.kind != PP_KIND_FFT ||
+        need <= std::min(h->bufA.bytes, h->bufB.bytes))
+        return;
+    DevBuf A, B;
+    if (A.alloc(need) == cudaSuccess && B.alloc(need) == cudaSuccess) {
+        std::swap(h->bufA, A);
+        std::swap(h->bufB, B);
+    }
+    cudaGetLastError();
+    A.free();  // (waits for solves that still use them)
+    B.free();
 }
 
 // lines per tile of the generic transform kernel: the tuned value when it fits
@@ -1232,9 +1260,9 @@ int pp_create(int nx, int ny, int nz, pp_handle* out)
     *out = nullptr;
     pp_solver_s* h = nullptr;
     if (const int rc = new_handle(nx, ny, nz, &h)) return rc;
-    const size_t bytes = pp_spectrum_bytes(nx, ny, nz), grid = 2 * sizeof(double) * (size_t)nx * ny * nz;
-    if (h->rhs.alloc(grid) != cudaSuccess || h->bufA.alloc(bytes) != cudaSuccess ||
-        h->bufB.alloc(bytes) != cudaSuccess || h->out.alloc(grid) != cudaSuccess) {
+    const size_t grid = 2 * sizeof(double) * (size_t)nx * ny * nz;
+    if (h->rhs.alloc(grid) != cudaSuccess || h->bufA.alloc(grid) != cudaSuccess ||
+        h->bufB.alloc(grid) != cudaSuccess || h->out.alloc(grid) != cudaSuccess) {
         // release what did fit (the buffers have no destructor)
         h->rhs.free();
         h->bufA.free();
@@ -1299,6 +1327,7 @@ int pp_assign_boundary(pp_handle h, const char bc[6])
     std::memcpy(h->bc, bc, 6);
     int rc = rebuild_tables(h);
     h->have_bc = rc == PP_SUCCESS;
+    if (h->have_bc) grow_spectra(h);
     return rc;
 }
 
@@ -1947,17 +1976,18 @@ int pp_autotune(pp_handle h, int reps, pp_tuning* chosen, double* best_ms)
 
 }  // extern "C"
 
-size_t pp_spectrum_bytes(int nx, int ny, int nz)
+size_t pp_spectrum_bytes(int nx, int ny, int nz, bool y_periodic)
 {
-    return 2 * sizeof(double) * (size_t)(nx + pp_spare_cols(nx)) * ny * nz;
+    return 2 * sizeof(double) * (size_t)(nx + (y_periodic ? pp_spare_cols(nx) : 0)) * ny * nz;
 }
 
-int pp_create_lent(int nx, int ny, int nz, void* spec_a, void* spec_b, void* work, pp_solver_s** out)
+void pp_allow_padding(pp_solver_s* h, bool allow) { h->may_pad = allow; }
+
+int pp_create_lent(int nx, int ny, int nz, void* spec_a, void* spec_b, size_t bytes, void* work, pp_solver_s** out)
 {
     *out = nullptr;
     pp_solver_s* h = nullptr;
     if (const int rc = new_handle(nx, ny, nz, &h)) return rc;
-    const size_t bytes = pp_spectrum_bytes(nx, ny, nz);
     h->bufA.borrow(spec_a, bytes);
     h->bufB.borrow(spec_b, bytes);
     h->out.borrow(work, work ? bytes / 4 : 0);
