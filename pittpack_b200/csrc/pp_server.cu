@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "../../include/pittpack_b200.h"
+#include "pp_kernels.h"
 
 namespace {
 
@@ -125,7 +126,8 @@ PooledHandle* acquire(pp_server_s* S, const pp_request& r, const ShapeKey& key, 
         if (!handle_busy(S, &ph)) return &ph;
         have_shape = true;
     }
-    // a handle holds four 2-complex-per-point buffers plus tables
+    // a handle holds four buffers of a complex number per point, plus tables; the
+    // padding of a complex spectrum (a periodic y) only where there is room for it
     const size_t need = (size_t)r.nx * r.ny * r.nz * 8 * sizeof(double) + (1u << 20);
     if (have_shape && S->pool_bytes + need > S->budget) return nullptr;
     while (S->pool_bytes + need > S->budget) {
@@ -148,6 +150,8 @@ PooledHandle* acquire(pp_server_s* S, const pp_request& r, const ShapeKey& key, 
     }
     pp_handle h = nullptr;
     if ((*rc = pp_create(r.nx, r.ny, r.nz, &h)) != PP_SUCCESS) return nullptr;
+    const size_t spare = 2 * (pp_spectrum_bytes(r.nx, r.ny, r.nz, true) - pp_spectrum_bytes(r.nx, r.ny, r.nz, false));
+    pp_allow_padding(h, S->pool_bytes + need + spare <= S->budget);
     if ((*rc = pp_set_box(h, r.box)) != PP_SUCCESS || (*rc = pp_assign_boundary(h, r.bc)) != PP_SUCCESS) {
         pp_destroy(h);
         return nullptr;
