@@ -1,6 +1,6 @@
-// Transform pass for line lengths N = 16 .. 2048, powers of two (the real
-// families and half spectra of N = 32 .. 1024 take pp_rhalf.cuh, so that those
-// lengths are here for complex lines): the same four passes and the same
+// Transform pass for line lengths N = 16 .. 2048, powers of two: complex lines of
+// each, the real families of 16 and 2048 and the half spectra of 2048 (those of
+// N = 32 .. 1024 take pp_rhalf.cuh): the same four passes and the same
 // per-family pre/post-processing as pp_linepass.cu (see the reference
 // citations there), built on the register-resident FFT of pp_fftreg.cuh and
 // specialised at compile time on the length and the boundary family, so that
@@ -19,8 +19,8 @@
 // pass a row segment of the tile's lines); (2) each thread gathers its pass-0
 // FFT inputs from the raw tile with the family's reorder folded into the
 // addresses (radix 8 first, so which half a register falls in is known at
-// compile time); (3) FFT, ending with the radix-m pass where m > 1;
-// (4) post-processing of pairs (k, N-k), each Z read once, and stores.  The
+// compile time); (3) FFT; (4) post-processing of pairs (k, N-k), each Z read
+// once, and stores.  The
 // forward x pass's dz^2 scaling is applied to the
 // outputs (a linear factor), the Dirichlet lift is subtracted (divided by
 // dz^2) from the few raw elements on a Dirichlet face.
@@ -35,7 +35,7 @@
 
 namespace pp_lp2 {
 
-// F_R2C / F_C2R: the periodic x pass of a real RHS on half spectra (k <= N/2,
+// F_R2C / F_C2R: the periodic (contiguous) x pass of a real RHS on half spectra (k <= N/2,
 // the other half is the conjugate mirror): two real lines per complex FFT
 enum Fam : int { F_DST2 = 0, F_DCT2 = 1, F_FFT = 2, F_Q4 = 3, F_R2C = 4, F_C2R = 5 };
 
@@ -329,8 +329,7 @@ __device__ __forceinline__ void lp2_body(const PPLinePassArgs& a)
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const int m = t + q * (N / 8);
-            if (STRIDED) v[q] = *reinterpret_cast<const C*>(raw + ridx(la, m));
-            else v[q] = mkc<C>(raw[ridx(la, m)], raw[ridx(lb, m)]);
+            v[q] = mkc<C>(raw[ridx(la, m)], raw[ridx(lb, m)]);
         }
     } else if constexpr (C2R) {
         // Z_m = X_a,m + i X_b,m with the upper half rebuilt as the conjugate
@@ -469,16 +468,8 @@ __device__ __forceinline__ void lp2_body(const PPLinePassArgs& a)
     } else if constexpr (R2C) {
         // half spectra k = 0..N/2 of both packed lines:
         // X_a,k = (Z_k + conj Z_{N-k}) / 2, X_b,k = (Z_k - conj Z_{N-k}) / (2i)
-        constexpr int LL = rp_log2(LPC);
         for (int idx = tid; idx < LPC * (N / 2); idx += NT) {
-            int cl, kk;
-            if (STRIDED) {
-                cl = idx & (LPC - 1);
-                kk = idx >> LL;
-            } else {
-                cl = idx / (N / 2);
-                kk = idx - cl * (N / 2);
-            }
+            const int cl = idx / (N / 2), kk = idx - cl * (N / 2);
             const int la = 2 * cl, lb = la + 1;
             const C* ln = sb + cl * P1;
             auto emit = [&](int k, C Zk, C Zn) {
@@ -507,16 +498,8 @@ __device__ __forceinline__ void lp2_body(const PPLinePassArgs& a)
         }
     } else if constexpr (C2R) {
         // z = x_a + i x_b: both real lines at once
-        constexpr int LL = rp_log2(LPC);
         for (int idx = tid; idx < LPC * N; idx += NT) {
-            int cl, e;
-            if (STRIDED) {
-                cl = idx & (LPC - 1);
-                e = idx >> LL;
-            } else {
-                cl = idx / N;
-                e = idx - cl * N;
-            }
+            const int cl = idx / N, e = idx - cl * N;
             const int la = 2 * cl, lb = la + 1;
             const C z = sb[cl * P1 + rp_pad(e)];
             if (la < nl) put<Real>(a, goff(la, e), plane, z.x, (Real)0, sc);
@@ -590,13 +573,7 @@ __device__ __forceinline__ void lp2_body(const PPLinePassArgs& a)
         constexpr int LL = rp_log2(LPC);
         for (int idx = tid; idx < LPC * N; idx += NT) {
             int cl, e;
-            if (STRIDED && LPC == 4) {
-                // an 8-thread phase takes outputs e, e + 2 of four lines: their
-                // spectrum slots are adjacent (8 distinct banks)
-                cl = idx & 3;
-                const int rest = idx >> 3;
-                e = 4 * (rest >> 1) + (rest & 1) + 2 * ((idx >> 2) & 1);
-            } else if (STRIDED) {
+            if (STRIDED) {
                 cl = idx & (LPC - 1);
                 e = idx >> LL;
             } else {
@@ -677,8 +654,10 @@ cudaError_t launch_n(const PPLinePassArgs& a, bool inverse, bool strided, cudaSt
                                                 : cudaErrorInvalidValue;
     } else {
     if (a.half && a.kind == PP_KIND_FFT) {
-        if (strided) return cudaErrorInvalidValue;
-        return inverse ? launch_half<Real, N, LPC, F_C2R>(a, st) : launch_half<Real, N, LPC, F_R2C>(a, st);
+        if constexpr (N >= 32)
+            if (!strided)
+                return inverse ? launch_half<Real, N, LPC, F_C2R>(a, st) : launch_half<Real, N, LPC, F_R2C>(a, st);
+        return cudaErrorInvalidValue;
     }
     switch (a.kind) {
     case PP_KIND_DST2: return launch_fam<Real, N, LPC, F_DST2>(a, inverse, strided, st);
