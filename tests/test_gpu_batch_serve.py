@@ -79,6 +79,38 @@ def test_batch_graph_matches_single_solves(precision):
     B.close()
 
 
+@pytest.mark.parametrize("order", [1, -1])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_one_branch_runs_unlike_grids_in_one_workspace(precision, order):
+    """Large and tiny grids, real, complex, half and padded spectra take the same
+    buffers in turn: none may depend on what an earlier one left there."""
+    import torch
+
+    from pittpack_b200.batch import Batch
+
+    shapes = [(160, 128, 100, "NNPPDD"), (16, 18, 9, "DDDDNN"), (100, 96, 60, "NDDDDN"), (64, 64, 64, "PPPPNN"),
+              (50, 42, 37, "NNDDNN"), (100, 64, 33, "DDPPDD"), (32, 32, 200, "NNNNDD"), (7, 11, 5, "PPPPDD")]
+    grids = []
+    for k, (nx, ny, nz, bc) in enumerate(shapes[::order]):
+        f = np.random.default_rng(k).standard_normal((nz, ny, nx))
+        grids.append((nx, ny, nz, bc, f - f.mean() if "D" not in bc else f))
+    bufs = [(torch.from_numpy(f.ravel().copy()).cuda(), torch.empty(2 * f.size, dtype=torch.float64, device="cuda"))
+            for *_, f in grids]
+    B = Batch([dict(nx=nx, ny=ny, nz=nz, bc=bc, d_rhs=r.data_ptr(), d_P=P.data_ptr())
+               for (nx, ny, nz, bc, _), (r, P) in zip(grids, bufs)], precision=precision, sweeps=2, branches=1,
+              autotune=False)
+    for _ in range(2):
+        for _, P in bufs:
+            P.zero_()
+        torch.cuda.synchronize()
+        B.run(torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        for grid, (_, P) in zip(grids, bufs):
+            nx, ny, nz = grid[:3]
+            _check(P.cpu().numpy().view(np.complex128).reshape(nz, ny, nx), grid, precision)
+    B.close()
+
+
 def test_server_results_same_alone_and_in_the_mix():
     from pittpack_b200.batch import Server
     from pittpack_b200.poisson import pinned_empty

@@ -39,6 +39,30 @@ def test_lanes(nz, bc):
         assert M.kernelTimeouts() == 0
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("bc", ["NNNNDD", "NDNDPP", "DDNDDN", "NNPPNN"])
+@pytest.mark.parametrize("nz", NZ)
+def test_bulk_tiles(nz, bc, precision):
+    # ny = 64: the y pass has 8 lines a tile, real spectra too, so that the lanes
+    # that leave a CTA its 8 systems copy their blocks of rows in bulk
+    import pittpack_b200 as pp
+
+    nx, ny = 24, 64
+    f = _rhs((nz, ny, nx), nz, bc)
+    Q = O.solve(O.problem(nx, ny, nz, bc, compat_zero_mode=1 - precision), f)
+    with pp.make_Poisson(nx, ny, nz) as M:
+        M.setOptions(precision=precision, max_sweeps=3, compat_zero_mode=1 - precision)
+        M.assignBoundary(bc)
+        M.assignRhs(f)
+        for lanes in (0, 1, 2, 4, 8, 16, 32):
+            if lanes > 1 and lanes > nz // 2:
+                continue
+            M.setTuning(zsolve_lanes=lanes)
+            M.pittPack()
+            assert O.rel_l2(M.getSolution().real, Q.real) <= (1e-10 if precision else 1e-12), lanes
+        assert M.kernelTimeouts() == 0
+
+
 @pytest.mark.parametrize("bc", ["NNNNDD", "PPPPPP", "NDPPDN"])
 @pytest.mark.parametrize("nz", [9, 19, 25, 37, 50, 75, 129])
 def test_refined(nz, bc):
