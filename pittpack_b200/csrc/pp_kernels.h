@@ -32,10 +32,11 @@ struct PPLinePassArgs {
     long elem_stride;  // strides in elements (complex elements count once)
     long line_stride;
     long plane_stride;
-    // power-of-two kernel only: the tile of lines l0.. starts at
+    // every kernel but the generic one: the tile of lines l0.. starts at
     // plane * plane_stride + l0 * tile_stride (0: l0 * line_stride), and the
     // output may use its own strides (o_*; o_elem_stride = 0: the input's).
-    // This lets the y passes write / read the z-tiled spectrum layout.
+    // This lets the y passes write / read the z-tiled spectrum layout, and the x
+    // passes rows of their own width (half spectra, padded rows).
     long tile_stride;
     long o_elem_stride, o_line_stride, o_plane_stride, o_tile_stride;
     int L;             // lines per CTA tile
@@ -47,16 +48,17 @@ struct PPLinePassArgs {
     PPLift lift;
     int nx, ny, nz;
     double out_scale;  // inverse x-pass: 1 / (nx ny)
-    // twiddles in the kernel's precision: used by the power-of-two kernel
-    // (pp_linepass_pow2.cu) and by the FP32 generic kernel
+    // twiddles in the kernel's precision: used by the tile kernel (pp_lp2.cuh), the
+    // half-length and planned ones (pp_rhalf.cuh, pp_mr.cuh) and the FP32 generic one
     const void* tw;    // FFT twiddles (double2 or float2), length n or n/2
     const void* cs2;   // family twiddles in the kernel's precision
     int in_cplx, out_cplx;
-    int vec16;          // power-of-two kernel: src and its run starts are 16-byte aligned
-                        // (half-length kernel: aligned to its widest load)
-    int vec_out;        // half-length kernel: dst and its runs are aligned to its widest store
-    int half;           // power-of-two periodic x pass of a real RHS on half spectra
-                        // (N/2 + 1 complex per line): forward real -> half, inverse half -> real
+    int vec16;          // tile kernel: src and its run starts are 16-byte aligned
+                        // (half-length and planned kernels: aligned to the widest load)
+    int vec_out;        // half-length and planned kernels: dst and its runs are aligned to the widest store
+    int half;           // periodic x pass of a real RHS on half spectra (N/2 + 1 complex per
+                        // line): forward real -> half, inverse half -> real (read as reals
+                        // where in_cplx is 0, after a non-periodic y)
     // refinement epilogue of the inverse x pass (acc != null): the real part v
     // of each output becomes u = acc + out_scale v + zplane[plane] in FP64;
     // written to acc, or (dst != null) as the final complex-interleaved P

@@ -1,5 +1,7 @@
 // Transform pass for line lengths other than powers of two whose FFT factors into
-// 2, 3, 5, 7, 11 and 13, by a plan of radices.
+// 2, 3, 5, 7, 11 and 13, by a plan of radices: up to 4096 FFT points, less 46
+// counts from 2860 on (2970, 3240, 3456, ..) that would need more butterflies a
+// thread than its registers take and stay with the generic kernel.
 //
 // The same per-family pre/post-processing as pp_linepass.cu (see the reference
 // citations there), on the fewest complex points:
@@ -15,13 +17,16 @@
 // the pre-processing folded in (a thread forms the pair k, M - k of the
 // inverse transforms); (2) Stockham passes in place, of radix up to 20: every
 // thread reads its butterflies into registers, the CTA meets, and writes them
-// back, so that M <= 320 takes two passes and M <= 6400 three; (3) FFT output
-// -> global memory with the post-processing.
+// back: two passes where M is a product of two such radices (107 of the 125
+// counts up to 320, and 324, 360, 400), else three (125, 147, 243, 250, 500, ..),
+// four for 40 counts from 625 on; (3) FFT output -> global memory with the
+// post-processing.
 //
 // The lengths that people choose (pp_mr_ct_*.cu: the decimal edges 50, 60, 100,
 // 200, 300, 500, 1000, the multiples 48, 96, 144, 192, 288, 384, 576, 768 and
-// their like) are instances with the plan known at compile time; the others take
-// one kernel that reads it at run time, its passes functions of their own.
+// their like, even and of factors 2, 3 and 5) are instances with the plan known at
+// compile time; the others take one kernel that reads it at run time, its passes
+// functions of their own.
 //
 // What bounds it is the shared-memory pipe (about 8 + 8 + 16 passes + 8 + 8 bytes
 // a point, 50 - 68 % busy), then the latency of the phases at 14 to 20 warps
@@ -30,7 +35,7 @@
 // solve, before (pp_linepass.cu; * a register kernel for m 2^k) -> run-time plan
 // -> compile-time plan:
 //   200^3 N-N            0.888 -> 0.34 -> 0.189    384^3 N-N *  1.25 -> 1.08
-//   500 x 400 x 300 D-D  6.48      ->     1.41     192^3 P-P *  0.184 -> 0.152
+//   500 x 400 x 300 D-D  6.48      ->     1.34     192^3 P-P *  0.184 -> 0.152
 //   1000 x 800 x 100     9.06  -> 4.2  -> 1.78     960^2 x 128 * 5.05 -> 3.52
 // The generic kernel of before (one complex FFT of N per real line, radix <= 8 in
 // two ping-pong buffers, half a dozen passes over them) stays for larger prime

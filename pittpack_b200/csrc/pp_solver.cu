@@ -680,13 +680,6 @@ void set_rows_in(PPLinePassArgs& a, bool half, int ncol, long splane, int nx, lo
     a.o_tile_stride = 0;
 }
 
-// Width of the z-tiled spectrum layout for this solve, 0 for the usual one.
-// The forward y pass writes, and the inverse y pass reads, the spectrum as
-// contiguous z tiles (TS adjacent kx x all nz of one ky), so that the z solve
-// moves whole contiguous blocks; TS is the y pass's lines per tile.  Used
-// when the y pass takes strides of its own (every kernel but the generic one)
-// with full tiles (the columns a multiple of TS), the z solve is the direct one
-// and takes TS systems per CTA.
 // data lines per tile of the y pass (0: the generic kernel)
 int y_tile_lines(const DirTables& t)
 {
@@ -695,12 +688,23 @@ int y_tile_lines(const DirTables& t)
     if (const int lpc = pp_lp2_lpc(t.n)) return cplx ? lpc : 2 * lpc;
     return t.mr.m ? pp_mr_lines(t.n, t.kind, t.mr) : 0;
 }
+// Width of the z-tiled spectrum layout for this solve, 0 for the usual one.
+// The forward y pass writes, and the inverse y pass reads, the spectrum as
+// contiguous z tiles (TS adjacent kx x all nz of one ky), so that the z solve
+// moves whole contiguous blocks; TS is the y pass's lines per tile.  Used
+// when the y pass takes strides of its own (every kernel but the generic one)
+// with full tiles (the columns a multiple of TS), the z solve is the direct one
+// and takes TS systems per CTA.
 int z_tile_width(const pp_solver_s* h, bool s_cplx, int ncol)
 {
     if (h->opt.z_solver != PP_ZSOLVE_DIRECT || h->slab) return 0;
     const int dl = y_tile_lines(h->ty);
-    // (rows of at least 64 bytes: on narrower ones the z solve's tiles are worth
-    // less than its own row segments, 1280 x 1280 x 64 periodic 0.85 and 0.49 ms)
+    // (rows of at least 64 bytes: narrower ones are worth less than the z solve's own
+    // row segments, and cost the y passes.  z tiles and segments, ms: 1280 x 1280 x 64
+    // periodic, z 0.85 and 0.49; complex y of 1024 points, two lines a tile: 1024 x 1024
+    // x 64 N-N z 1.04 and 0.59, forward y 0.89 and 0.82, 1024 x 1024 x 128 complex z
+    // 1.37 and 1.21, y 1.73 and 1.41, 512 x 1024 x 128 P-P z 0.295 and 0.309, y 0.367
+    // and 0.329)
     if (dl * (s_cplx ? 16 : 8) < 64 || dl > 16 || ncol % dl != 0) return 0;
     if (h->tune.zsolve_tile != 0 && h->tune.zsolve_tile != dl) return 0;
     int ts = 0, threads = 0;
@@ -729,10 +733,10 @@ int half_spectrum_cols(const pp_solver_s* h)
 // pass's lines per tile where that costs at most an eighth more: full tiles let
 // the z solve take the z-tiled layout, and rows of 64 bytes start on 32-byte
 // sectors (500 x 400 x 300 D-D, 500 -> 504 columns: z solve 0.382 -> 0.293 ms, the
-// transform passes as before).  The padding columns are zeros throughout.  Only where the x pass
-// writes rows of their own stride (the planned kernel: every other one's nx is
-// a multiple already, or has no strides of its own), not for slabs or the
-// alternate z solvers, and only as far as the spectrum buffers reach.
+// transform passes as before).  The padding columns are zeros throughout.  Only
+// where the x pass writes rows of their own stride (the planned kernel: every
+// other one's nx is a multiple already, or has no strides of its own), not for
+// slabs or the alternate z solvers, and only as far as the spectrum buffers reach.
 int padded_cols(const pp_solver_s* h)
 {
     const int q = y_tile_lines(h->ty);

@@ -29,8 +29,8 @@
 //     rows stay in registers where the counts allow.  Interior rows have the
 //     same coefficients in every block, so the pivots and spikes of a block
 //     depend only on lambda; the CTA builds them into a shared table (one
-//     reciprocal per entry) that every lane reads, and the sweeps divide only
-//     on the system's last row;
+//     reciprocal per entry) that every lane reads, and the sweeps do not
+//     divide: the system's first and last rows scale their blocks' ends;
 //   * eliminating each lane's first unknown leaves a P-row tridiagonal system
 //     in the lanes' last unknowns, solved by parallel cyclic reduction over
 //     warp shuffles (on the ring of lanes for periodic systems); each lane
@@ -812,8 +812,8 @@ __global__ void __launch_bounds__(PP_Z_THREADS) zsolve_kernel(PPZArgs a)
 // The split kernels held to 128 registers (two CTAs of 256 threads, or four
 // of 128, per SM): their sweeps are bound by the latency of dependent FP64
 // operations, and the extra resident warps outweigh a few spilled values
-// (512^3: real 32 rows per lane 0.436 -> 0.380 ms with 92 bytes spilled,
-// complex 16 rows 0.446 -> 0.381 ms; FP32 complex spectra 0.37 -> 0.33 ms).
+// (512^3: real 32 rows per lane 0.436 -> 0.380 ms, complex 16 rows 0.446 ->
+// 0.381 ms, 40 to 50 bytes spilled each; FP32 complex spectra 0.37 -> 0.33 ms).
 // Not for FP32 real spectra, whose conversions make the cap cost more than
 // it gains (0.33 -> 0.36 ms).  A separate kernel: naming a minimum of one
 // CTA per SM in the other kernels' launch bounds lets the compiler spend
@@ -834,6 +834,7 @@ void (*split_kernel())(PPZArgs)
 
 int pp_zsolve_lanes(int nz, bool cplx, long systems)
 {
+    // (the error does not depend on the lanes: rows are carried by their sums)
     // the fewest lanes that keep every lane's rows in registers: fewer lanes mean
     // fewer steps of the reduced system's PCR per row (384 x 384 x 272, real: 8
     // lanes of 34 rows 0.164 ms, 16 of 17 0.209; 192 x 160 x 144, complex: 8 of 18
