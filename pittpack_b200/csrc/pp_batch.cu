@@ -91,7 +91,8 @@ int build_handles(pp_batch_s* b, const pp_batch_item* items, int n, const pp_opt
         size_t bytes = 0;
         for (int i = k; i < n; i += branches) {
             const pp_batch_item& it = items[i];
-            if (it.nx > 0 && it.ny > 0 && it.nz > 0)
+            // (grids that pp_create refuses get their own error below)
+            if (it.nx >= 2 && it.ny >= 2 && it.nz >= 3 && it.nz <= pp_zsolve_max_nz(false, false))
                 bytes = std::max(bytes, pp_spectrum_bytes(it.nx, it.ny, it.nz, it.bc[2] == 'P'));
         }
         const size_t want[3] = {bytes, bytes, refined ? bytes / 4 : 0};

@@ -79,6 +79,23 @@ def test_batch_graph_matches_single_solves(precision):
     B.close()
 
 
+@pytest.mark.parametrize("nx,ny,nz,code", [(1, 200000, 200000, 19), (100000, 100000, 2, 19), (2000, 2000, 30000, 27)])
+def test_refused_grids_keep_their_codes(nx, ny, nz, code):
+    # sizes that no handle takes are refused as such, not for the memory they would need
+    import torch
+
+    import pittpack_b200 as pp
+    from pittpack_b200.batch import Batch
+
+    with pytest.raises(pp.PittPackError) as e:
+        pp.make_Poisson(nx, ny, nz)
+    assert e.value.code == code
+    d = torch.zeros(16, dtype=torch.float64, device="cuda")
+    with pytest.raises(pp.PittPackError) as e:
+        Batch([dict(nx=nx, ny=ny, nz=nz, bc="NNNNDD", d_rhs=d.data_ptr(), d_P=d.data_ptr())], autotune=False)
+    assert e.value.code == code
+
+
 @pytest.mark.parametrize("order", [1, -1])
 @pytest.mark.parametrize("precision", [0, 1])
 def test_one_branch_runs_unlike_grids_in_one_workspace(precision, order):
