@@ -86,9 +86,36 @@ struct PPMrPlan {
 bool pp_mr_plan(int n, int kind, bool half, PPMrPlan* p);
 // data lines per CTA tile
 int pp_mr_lines(int n, int kind, const PPMrPlan& p);
-// one pass (a.tw and a.cs2 in its precision, strides and output strides set)
+// one pass (a.tw and a.cs2 in its precision, strides and output strides set), in
+// this kernel or where it is faster in the register kernel below
 cudaError_t pp_mr_line_pass(PPLinePassArgs a, const PPMrPlan& p, bool inverse, bool strided, bool in_cplx,
                             bool out_cplx, bool fp32, cudaStream_t st);
+// Whether a contiguous FP64 pass of a planned length runs the register kernel of
+// the lengths m 2^k instead (lpm_kernel, pp_lp2.cuh).  From 480 FFT points on the
+// planned kernel's tiles of up to 4096 points leave a CTA two to four lines (two-way
+// bank conflicts below eight) and an SM two or three CTAs.  Planned and register
+// kernel, us a pass over 24 M points, 128 rows a plane:
+//   complex   480 250 and 195, 576 235 and 170, 640 237 and 208, 768 224 and 210,
+//             960 232 and 183, 1152 252 and 195, 1536 281 and 215; 320 (16 M points)
+//             125 and 116, but 384 142 and 152
+//   half      forward 960 148 and 103, 1280 142 and 118, 1536 130 and 117, but 768
+//             105 and 117; inverse 960 156 and 119, 1536 159 and 136
+//   N-N       forward 960 144 and 116, 1152 143 and 121, 1536 138 and 132, but 768
+//             114 and 117; inverse 576 136 and 122, 768 157 and 132, 960 183 and 134,
+//             1536 167 and 144, but 640 120 and 127 (D-D alike)
+// Strided, DCT-IV / DST-IV and FP32 passes are faster planned (y at 960^2 x 34 N-N 197
+// and 458 us; DST-IV 960 forward 152 and 146, inverse 170 and 201).  One line a CTA
+// in the planned kernel, odd radix first, did not reach it (960 N-N 125 and 161 us).
+constexpr bool pp_lpm_takes(int n, int kind, bool half, bool inverse)
+{
+    const bool large = n == 960 || n == 1152 || n == 1280 || n == 1536;
+    if (kind == PP_KIND_FFT && !half) return large || n == 320 || n == 480 || n == 576 || n == 640 || n == 768;
+    if (kind == PP_KIND_FFT) return large;
+    if (kind == PP_KIND_DST2 || kind == PP_KIND_DCT2) return large || (inverse && (n == 576 || n == 768));
+    return false;
+}
+cudaError_t pp_launch_lpm_cplx(const PPLinePassArgs& a, bool inverse, cudaStream_t st);
+cudaError_t pp_launch_lpm_real(const PPLinePassArgs& a, bool inverse, cudaStream_t st);
 cudaError_t pp_launch_mr_real_f64(const PPLinePassArgs& a, const PPMrPlan& p, bool inverse, bool strided, cudaStream_t st);
 cudaError_t pp_launch_mr_real_f32(const PPLinePassArgs& a, const PPMrPlan& p, bool inverse, bool strided, cudaStream_t st);
 cudaError_t pp_launch_mr_periodic_f64(const PPLinePassArgs& a, const PPMrPlan& p, bool inverse, bool strided,

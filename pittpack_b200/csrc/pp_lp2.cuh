@@ -1,6 +1,9 @@
 // Transform pass for line lengths N = 16 .. 2048, powers of two: complex lines of
 // each, the real families of 16 and 2048 and the half spectra of 2048 (those of
-// N = 32 .. 1024 take pp_rhalf.cuh): the same four passes and the same
+// N = 32 .. 1024 take pp_rhalf.cuh); and for the contiguous (x) passes of the
+// lengths m 2^k (m = 3, 5, 9, 15) that pp_lpm_takes lists, whose power-of-two
+// factor runs as register passes and the odd one as a last Stockham pass of
+// radix m and span 2^k in shared memory: the same four passes and the same
 // per-family pre/post-processing as pp_linepass.cu (see the reference
 // citations there), built on the register-resident FFT of pp_fftreg.cuh and
 // specialised at compile time on the length and the boundary family, so that
@@ -19,8 +22,8 @@
 // pass a row segment of the tile's lines); (2) each thread gathers its pass-0
 // FFT inputs from the raw tile with the family's reorder folded into the
 // addresses (radix 8 first, so which half a register falls in is known at
-// compile time); (3) FFT; (4) post-processing of pairs (k, N-k), each Z read
-// once, and stores.  The
+// compile time); (3) FFT, ending with the radix-m pass where m > 1; (4)
+// post-processing of pairs (k, N-k), each Z read once, and stores.  The
 // forward x pass's dz^2 scaling is applied to the
 // outputs (a linear factor), the Dirichlet lift is subtracted (divided by
 // dz^2) from the few raw elements on a Dirichlet face.
@@ -58,6 +61,46 @@ struct Vec2<float> {
 };
 
 PP_D int mk_pos(int e, int n) { return (e & 1) ? (n - 1 - (e >> 1)) : (e >> 1); }
+
+// R-point DFT in registers, R = 3 or 5 (pp_fft.cuh)
+template <int SIGN, int R, typename C>
+PP_D void small_dft(C* v)
+{
+    if constexpr (R == 3) dft3<SIGN>(v);
+    else dft5<SIGN>(v);
+}
+
+// MM = A B point DFT by one Cooley-Tukey step: n = B n1 + n2, k = k1 + A k2;
+// A-point DFTs over n1, twiddles W_MM^{n2 k1}, B-point DFTs over n2.  W_MM^x
+// is taken from the FFT's own table as tw[x * stride] (stride = NF / MM).
+template <int SIGN, int A, int B, typename C>
+PP_D void dft_ct(C* v, const C* __restrict__ tw, int stride)
+{
+    C y[B][A];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) {
+#pragma unroll
+        for (int n1 = 0; n1 < A; ++n1) y[n2][n1] = v[B * n1 + n2];
+        small_dft<SIGN, A>(y[n2]);
+    }
+#pragma unroll
+    for (int n2 = 1; n2 < B; ++n2)
+#pragma unroll
+        for (int k1 = 1; k1 < A; ++k1) {
+            C w = __ldg(&tw[n2 * k1 * stride]);
+            if (SIGN > 0) w.y = -w.y;
+            y[n2][k1] = c_mul(y[n2][k1], w);
+        }
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) {
+        C z[B];
+#pragma unroll
+        for (int n2 = 0; n2 < B; ++n2) z[n2] = y[n2][k1];
+        small_dft<SIGN, B>(z);
+#pragma unroll
+        for (int k2 = 0; k2 < B; ++k2) v[k1 + A * k2] = z[k2];
+    }
+}
 
 PP_D double lift_at(const PPLift& L, int i, int j, int k, int nx, int ny, int nz)
 {
@@ -313,8 +356,11 @@ __device__ __forceinline__ void lp2_body(const PPLinePassArgs& a)
     // radix 8 first: register q holds point m = t + q N/8 (t < N/8), so the
     // half of the line it falls in is known from q at compile time
     constexpr int NF = Q4 ? N / 2 : N;  // FFT length
+    constexpr int MF = rp_pow2_part(NF);  // its power-of-two factor (register passes)
+    constexpr int MM = NF / MF;           // and its odd factor (one radix-MM pass)
+    static_assert(MM == 1 || MM == 3 || MM == 5 || MM == 9 || MM == 15, "FFT length 2^k, 3 2^k, 5 2^k, 9 2^k or 15 2^k");
     constexpr int TPL = NF / 8;         // threads per FFT line
-    static_assert(rp_radix(NF, 0) == 8, "the first pass is radix 8");
+    static_assert(rp_radix(MF, 0) == 8, "the first pass is radix 8");
     static_assert(!(FAM == F_DST2 && INVERSE) || TPL % 2 == 0, "the DST-III sign uses the parity of t");
     const int fl = tid / TPL;           // FFT line of this thread
     const int t = tid - fl * TPL;
@@ -418,10 +464,48 @@ __device__ __forceinline__ void lp2_body(const PPLinePassArgs& a)
     // ---- 3. FFT (its first exchange starts with a barrier, so the raw tile
     //         that aliases the line buffers is no longer needed) ----------------------
     constexpr int FS = (INVERSE && !Q4) ? +1 : -1;
-    rp_fft<FS, NF>(v, line, t, tw);
+    rp_fft<FS, NF, MF>(v, line, t, tw);
     __syncthreads();  // all reads of the last exchange are done
+    if constexpr (MM == 1) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) line[rp_pad(rp_out_index<NF>(t, j))] = v[j];
+        for (int j = 0; j < 8; ++j) line[rp_pad(rp_out_index<NF>(t, j))] = v[j];
+    } else {
+        // Stockham output of the last register pass, then the final pass of
+        // radix MM and span MF, in place: butterfly j < MF reads points
+        // j + q MF, multiplies point q by W_NF^{q j} and writes output q to
+        // j + q MF (natural order)
+        constexpr int NPM = rp_npass(MF);
+        rp_scatter<NF, rp_radix(MF, NPM - 1), rp_ns(MF, NPM - 1)>(v, line, t);
+        __syncthreads();
+        constexpr int NB = (MF + TPL - 1) / TPL;  // butterflies of this thread, at most
+        C u[NB][MM];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const int j = t + b * TPL;
+            if (j < MF) {
+#pragma unroll
+                for (int q = 0; q < MM; ++q) u[b][q] = line[rp_pad(j + q * MF)];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const int j = t + b * TPL;
+            if (j < MF) {
+#pragma unroll
+                for (int q = 1; q < MM; ++q) {
+                    C w = __ldg(&tw[q * j]);
+                    if (FS > 0) w.y = -w.y;
+                    u[b][q] = c_mul(u[b][q], w);
+                }
+                if constexpr (MM == 3 || MM == 5) small_dft<FS, MM>(u[b]);
+                else if constexpr (MM == 9) dft_ct<FS, 3, 3>(u[b], tw, MF);
+                else dft_ct<FS, 5, 3>(u[b], tw, MF);
+#pragma unroll
+                for (int q = 0; q < MM; ++q) line[rp_pad(j + q * MF)] = u[b][q];
+            }
+        }
+    }
     __syncthreads();
 
     // ---- 4. post-processing and stores ------------------------------------------------
@@ -598,6 +682,15 @@ __global__ void __launch_bounds__(LPC * N / 8) lp2_kernel(PPLinePassArgs a)
 {
     lp2_body<Real, N, LPC, FAM, INVERSE, STRIDED>(a);
 }
+// the lengths with an odd factor, whose final radix-m pass holds up to three
+// butterflies per thread: a register bound that leaves room for one more CTA per
+// SM (the second argument of __launch_bounds__ is what bounds the registers)
+constexpr int lpm_min_blocks(int nt) { return 65536 / (84 * nt) > 1 ? 65536 / (84 * nt) : 1; }
+template <typename Real, int N, int LPC, int FAM, bool INVERSE>
+__global__ void __launch_bounds__(LPC * N / 8, lpm_min_blocks(LPC * N / 8)) lpm_kernel(PPLinePassArgs a)
+{
+    lp2_body<Real, N, LPC, FAM, INVERSE, false>(a);
+}
 // the periodic family's 512-point FP64 instance (complex lines): bounded to 48
 // registers, five CTAs of 256 threads per SM (measured faster)
 template <typename Real, int N, int LPC, int FAM, bool INVERSE, bool STRIDED>
@@ -666,6 +759,18 @@ cudaError_t launch_n(const PPLinePassArgs& a, bool inverse, bool strided, cudaSt
     default: return launch_fam<Real, N, LPC, F_Q4>(a, inverse, strided, st);
     }
     }
+}
+
+// a contiguous pass of an odd multiple of a power of two (pp_lpm_*.cu)
+template <int N, int LPC, int FAM, bool INV>
+cudaError_t launch_lpm(const PPLinePassArgs& a, cudaStream_t st)
+{
+    constexpr size_t smem = smem_bytes<double, N, LPC, FAM, INV, false>();
+    auto kfn = lpm_kernel<double, N, LPC, FAM, INV>;
+    const cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kfn<<<a.nplanes * a.tiles_per_plane, LPC * N / 8, smem, st>>>(a);
+    return cudaGetLastError();
 }
 
 // lines per CTA (complex FFT lines) for a power-of-two length; 0 if the

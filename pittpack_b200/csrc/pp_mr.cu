@@ -57,6 +57,14 @@ cudaError_t pp_mr_line_pass(PPLinePassArgs a, const PPMrPlan& p, bool inverse, b
     auto whole = [](const void* q, long s1, long s2, size_t elem, size_t w) {
         return reinterpret_cast<uintptr_t>(q) % w == 0 && ((size_t)s1 * elem) % w == 0 && ((size_t)s2 * elem) % w == 0;
     };
+    if (!fp32 && !strided && pp_lpm_takes(a.n, a.kind, a.half, inverse)) {
+        // 16-byte runs of its input; lines a CTA as its launches have them, real ones two to an FFT
+        const int lpc = a.n >= 960 ? 1 : a.n >= 480 ? 2 : 4;
+        a.L = a.kind == PP_KIND_FFT && !a.half ? lpc : 2 * lpc;
+        a.tiles_per_plane = (a.nlines + a.L - 1) / a.L;
+        a.vec16 = whole(a.src, a.line_stride, a.plane_stride, (in_cplx ? 2 : 1) * es, 16);
+        return a.kind == PP_KIND_FFT ? pp_launch_lpm_cplx(a, inverse, st) : pp_launch_lpm_real(a, inverse, st);
+    }
     a.vec16 = !strided && !in_cplx && whole(a.src, a.line_stride, a.plane_stride, es, 2 * es);
     a.vec_out = !strided && whole(a.dst, own ? a.o_line_stride : a.line_stride, own ? a.o_plane_stride : a.plane_stride,
                                   (out_cplx ? 2 : 1) * es, (inverse ? 4 : 2) * es);

@@ -841,10 +841,17 @@ cudaError_t launch_kind(const PPLinePassArgs& a, const PPMrPlan& p, bool inverse
         kfn<<<a.nplanes * a.tiles_per_plane, p.threads, smem, st>>>(a, more...);
         return cudaGetLastError();
     };
-#define PP_MR(INV, STR)                                                    \
-    do {                                                                   \
-        if constexpr (M > 0) return go(mrc_kernel<Real, K, INV, STR, M>);  \
-        else return go(mr_kernel<Real, K, INV, STR>, p);                   \
+    // (contiguous FP64 passes that run the register kernel of pp_lp2.cuh have no instance here)
+    constexpr auto elsewhere = [](bool inv, bool str) constexpr {
+        const int n = K == K_CPLX ? M : 2 * M;
+        const int kind = K == K_REAL ? (int)PP_KIND_DCT2 : K == K_Q4 ? (int)PP_KIND_DCT4 : (int)PP_KIND_FFT;
+        return M > 0 && sizeof(Real) == 8 && !str && pp_lpm_takes(n, kind, K == K_HALF, inv);
+    };
+#define PP_MR(INV, STR)                                                                    \
+    do {                                                                                   \
+        if constexpr (elsewhere(INV, STR)) return cudaErrorInvalidValue;                   \
+        else if constexpr (M > 0) return go(mrc_kernel<Real, K, INV, STR, M>);             \
+        else return go(mr_kernel<Real, K, INV, STR>, p);                                   \
     } while (0)
     if constexpr (K == K_HALF) {
         if (strided) return cudaErrorInvalidValue;
