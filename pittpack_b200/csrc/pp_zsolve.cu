@@ -196,38 +196,31 @@ PP_D T zsolve_reduced(double ra, double rs, double rc, T rd, int lane, int P)
 //   E1: e1a f + l + e1c f_next = ..   alpha_k, gamma_k, the same sum.
 // A block that ends the system has no neighbour there, and its row is scaled:
 // by 1 / (psi_k - alpha_k) at a Neumann end (diagonal lambda + 1), by
-// 1 / (1 - gamma_k) at a Dirichlet one (lambda - 1).
-struct ZEnd {
-    double scale, c, sum;  // of the row: scale, coefficient across the block, sum
+// 1 / (1 - gamma_k) at a Dirichlet one (lambda - 1).  Selects, not branches: the
+// divisions of a lane's two ends overlap.
+struct ZRow {
+    double a, c, sum, scale;  // coefficients towards the neighbour and across the block, sum, scale
 };
-PP_D ZEnd zend(bool neumann, double g, double al, double psi)
+PP_D ZRow zend(bool end, bool neumann, double g, double al, double psi)
 {
-    ZEnd e;
-    e.scale = 1.0 / (neumann ? psi - al : 1.0 - g);
-    e.c = al * e.scale;
-    e.sum = neumann ? psi * e.scale : 1.0 + e.c;
-    return e;
+    ZRow r;
+    r.scale = 1.0 / (end ? (neumann ? psi - al : 1.0 - g) : 1.0);
+    r.a = end ? 0.0 : g;
+    r.c = al * r.scale;
+    r.sum = end && !neumann ? 1.0 + r.c : psi * r.scale;
+    return r;
 }
-// coefficients of E0 (q: the factor of its right-hand side d_0 - (row 1's)),
-// modified on the system's first block; pin: row 0 is x_0 = d_0, or
-// x_0 + x_{nz-1} = d_0 for periodic z
-struct ZFirst {
-    double a, c, sum, q;
-};
-PP_D ZFirst zfirst(bool first, bool pin, bool periodic, bool neumann, double g, double al, double psi)
+// E0, scale the factor of its right-hand side d_0 - (row 1's); pin: row 0 of the
+// system is x_0 = d_0, or x_0 + x_{nz-1} = d_0 for periodic z
+PP_D ZRow zfirst(bool first, bool pin, bool periodic, bool neumann, double g, double al, double psi)
 {
-    ZFirst r = {g, al, psi, g};
+    ZRow r = zend(first && !periodic, neumann, g, al, psi);
+    r.scale *= g;
     if (first && pin) {
         r.a = periodic ? 1.0 : 0.0;
         r.c = 0.0;
         r.sum = 1.0 + r.a;
-        r.q = 1.0;
-    } else if (first && !periodic) {
-        const ZEnd e = zend(neumann, g, al, psi);
-        r.a = 0.0;
-        r.c = e.c;
-        r.sum = e.sum;
-        r.q = g * e.scale;
+        r.scale = 1.0;
     }
     return r;
 }
@@ -288,17 +281,11 @@ PP_D void zsolve_split(T (&xr)[MT], const double2* tab, double psiA, double psiB
     }
     // ---- E0 and E1 of both blocks -------------------------------------------------------
     const double2 tA = tab[H - 1], tB = UNEV ? tab[HB - 1] : tA;
-    const ZFirst fa = zfirst(lane == 0, pin, periodic, nlo, tA.x, tA.y, psiA);
-    const T e0dA = zmul(fa.q, zsub(d0, lane == 0 && pin ? zzero<T>() : rA));
+    const ZRow fa = zfirst(lane == 0, pin, periodic, nlo, tA.x, tA.y, psiA);
+    const ZRow lb = zend(lane == P - 1 && !periodic, nhi, tB.x, tB.y, psiB);
+    const T e0dA = zmul(fa.scale, zsub(d0, lane == 0 && pin ? zzero<T>() : rA));
     const T e0dB = zmul(tB.x, zsub(live ? xr[H] : zzero<T>(), rB));
-    double e1aB = tB.y, e1cB = tB.x, e1sB = psiB;
-    if (lane == P - 1 && !periodic) {
-        const ZEnd e = zend(nhi, tB.x, tB.y, psiB);
-        e1aB = e.c;
-        e1cB = 0.0;
-        e1sB = e.sum;
-        dB = zmul(e.scale, dB);
-    }
+    dB = zmul(lb.scale, dB);
     // ---- rows of the blocks' last unknowns (off-diagonals and sums) ---------------------
     // l_A:  raA l_B(prev lane) + rbA l_A + rcA l_B = rdA
     const double raA = -tA.y * fa.a, rcA = -tA.x * tB.y, rsA = psiA - tA.y * fa.sum - tA.x * psiB;
@@ -307,8 +294,8 @@ PP_D void zsolve_split(T (&xr)[MT], const double2* tab, double psiA, double psiB
     const int nxt = (lane + 1) & (P - 1);
     const double nc0 = zshfl(fa.c, nxt, P), ns0 = zshfl(fa.sum, nxt, P);
     const T nd0 = zshfl(e0dA, nxt, P);
-    const double raB = -e1aB * tB.x, rcB = -e1cB * nc0, rsB = e1sB - e1aB * psiB - e1cB * ns0;
-    const T rdB = zsub(zsub(dB, zmul(e1aB, e0dB)), zmul(e1cB, nd0));
+    const double raB = -lb.c * tB.x, rcB = -lb.a * nc0, rsB = lb.sum - lb.c * psiB - lb.a * ns0;
+    const T rdB = zsub(zsub(dB, zmul(lb.c, e0dB)), zmul(lb.a, nd0));
     // l_A = pd - pa l_B(prev lane) - pc l_B, substituted into the l_B rows
     const double iA = 1.0 / (rsA - raA - rcA);
     const double pa = raA * iA, pc = rcA * iA, ps = rsA * iA;
@@ -509,6 +496,9 @@ PP_D void zsolve_body(PPZArgs a)
     double* bsc = reinterpret_cast<double*>(zsm_raw + Lz.red_off);
     const int mm = Lz.mmax;
     const int mcount = SPLIT ? MT / 2 : mm - 1;  // rows of the longest block: entries 1 .. mcount - 1
+    // block lengths of a launch: one where every lane has MT rows, else two (the
+    // split solve's second blocks and its first: three)
+    constexpr int NPSI = MT > 0 && !CAP ? 1 : SPLIT ? 3 : 2;
     // psi of the last row of the longest block, of one a row shorter (both in the
     // table's unused entry 0) and of one two rows shorter (past the scratch's u_i)
     auto psi_of = [&](int s, int j) -> double& {
@@ -527,7 +517,7 @@ PP_D void zsolve_body(PPZArgs a)
                 v += e * uc;
                 uc += v;
                 u[i] = uc;
-                if (i >= mcount - 3) psi_of(s, mcount - 1 - i) = w;  // (divided by u_i in phase 2)
+                if (i >= mcount - NPSI) psi_of(s, mcount - 1 - i) = w;  // (divided by u_i in phase 2)
             }
         } else {
             // q_i = 1 + t_i = 2 + e - 1 / q_{i-1}, t_i = e + t_{i-1} / q_{i-1};
@@ -539,7 +529,7 @@ PP_D void zsolve_body(PPZArgs a)
                 al *= p;
                 psi = (e + psi) * p;
                 tb[i] = make_double2(-p, al);
-                if (i >= mcount - 3) psi_of(s, mcount - 1 - i) = psi;
+                if (i >= mcount - NPSI) psi_of(s, mcount - 1 - i) = psi;
                 t = e + t * p;
             }
             u[0] = 0.0;
@@ -557,7 +547,7 @@ PP_D void zsolve_body(PPZArgs a)
             for (int i = (threadIdx.x & ((1 << ltp) - 1)) + 1; i < mcount; i += 1 << ltp) {
                 const double inv = -1.0 / u[i];
                 reinterpret_cast<double2*>(zsm_raw + Lz.tab_off)[(size_t)s * mm + i] = make_double2(u[i - 1] * inv, inv);
-                if (i >= mcount - 3) psi_of(s, mcount - 1 - i) *= -inv;
+                if (i >= mcount - NPSI) psi_of(s, mcount - 1 - i) *= -inv;
             }
     }
     cp_async_wait_all();
@@ -697,24 +687,17 @@ PP_D void zsolve_body(PPZArgs a)
             // in the lane's first (f) and last (l) unknowns
             const double2 tk = tab[M - 1];
             const double psi = psi_of(live ? s : 0, EXACT ? 0 : mcount - M);
-            const ZFirst fa = zfirst(lane == 0, pin, periodic, nlo, tk.x, tk.y, psi);
-            const double e0a = fa.a, e0c = fa.c;
-            const T e0d = zmul(fa.q, zsub(rD0, lane == 0 && pin ? zzero<T>() : dr));
-            double e1a = tk.y, e1c = tk.x, e1s = psi;
-            T e1d = dprev;
-            if (lane == P - 1 && !periodic) {
-                const ZEnd e = zend(nhi, tk.x, tk.y, psi);
-                e1a = e.c;
-                e1c = 0.0;
-                e1s = e.sum;
-                e1d = zmul(e.scale, e1d);
-            }
+            const ZRow fa = zfirst(lane == 0, pin, periodic, nlo, tk.x, tk.y, psi);
+            const ZRow lb = zend(lane == P - 1 && !periodic, nhi, tk.x, tk.y, psi);
+            const double e0a = fa.a, e0c = fa.c, e1a = lb.c, e1c = lb.a;
+            const T e0d = zmul(fa.scale, zsub(rD0, lane == 0 && pin ? zzero<T>() : dr));
+            const T e1d = zmul(lb.scale, dprev);
 
             // ---- reduced system ---------------------------------------------------------------
             // Eliminating every f_L with E0 leaves a tridiagonal system in l alone, one
             // row per lane (the Schur complement, an M-matrix with the original):
             //   -e1a e0a l_{L-1} + .. l_L - e1c e0c' l_{L+1} = e1d - e1a e0d - e1c e0d'
-            // of sum e1s - e1a e0s - e1c e0s'   (' : lane L+1)
+            // of the sum of E1's - e1a E0's - e1c E0's'   (' : lane L+1)
             // The lane indices wrap (periodic z); without it e0a = 0 on the first lane
             // and e1c = 0 on the last, so the wrapped values carry no weight.  It is
             // solved by parallel cyclic reduction over warp shuffles, and f_L follows
@@ -722,7 +705,7 @@ PP_D void zsolve_body(PPZArgs a)
             const int nxt = (lane + 1) & (P - 1);
             const double nc0 = zshfl(e0c, nxt, P), ns0 = zshfl(fa.sum, nxt, P);
             const T nd0 = zshfl(e0d, nxt, P);
-            const double ra = -e1a * e0a, rc = -e1c * nc0, rs = e1s - e1a * fa.sum - e1c * ns0;
+            const double ra = -e1a * e0a, rc = -e1c * nc0, rs = lb.sum - e1a * fa.sum - e1c * ns0;
             const T rd = zsub(zsub(e1d, zmul(e1a, e0d)), zmul(e1c, nd0));
             const T xl = zsolve_reduced(ra, rs, rc, rd, lane, P);
             const T xlp = zshfl(xl, (lane + P - 1) & (P - 1), P);
@@ -814,10 +797,12 @@ __global__ void __launch_bounds__(PP_Z_THREADS) zsolve_kernel(PPZArgs a)
 // operations, and the extra resident warps outweigh a few spilled values
 // (512^3: real 32 rows per lane 0.436 -> 0.380 ms, complex 16 rows 0.446 ->
 // 0.381 ms, 40 to 50 bytes spilled each; FP32 complex spectra 0.37 -> 0.33 ms).
-// Not for FP32 real spectra, whose conversions make the cap cost more than
-// it gains (0.33 -> 0.36 ms).  A separate kernel: naming a minimum of one
-// CTA per SM in the other kernels' launch bounds lets the compiler spend
-// more registers on them than the one-argument form does.
+// Not for FP32 real spectra of exact row counts, whose conversions make the cap
+// cost more than it gains (0.33 -> 0.36 ms); their uneven counts from 25 on take
+// it (512 x 512 planes, 27 rows 230 -> 187 us, 29 238 -> 191, 33 246 -> 201; FP64
+// 33 rows 133 -> 109).  A separate kernel: naming a minimum of one CTA per SM in
+// the other kernels' launch bounds lets the compiler spend more registers on them
+// than the one-argument form does.
 template <bool CPLX, bool G32, int MT, bool CAP>
 __global__ void __launch_bounds__(PP_Z_THREADS, 2) zsolve_split_r128_kernel(PPZArgs a)
 {
@@ -827,7 +812,7 @@ __global__ void __launch_bounds__(PP_Z_THREADS, 2) zsolve_split_r128_kernel(PPZA
 template <bool CPLX, bool G32, int MT, bool CAP>
 void (*split_kernel())(PPZArgs)
 {
-    if constexpr (CPLX ? MT <= 16 : (!G32 && MT <= 32)) return zsolve_split_r128_kernel<CPLX, G32, MT, CAP>;
+    if constexpr (CPLX ? MT <= 16 : (!G32 || (CAP && MT >= 26))) return zsolve_split_r128_kernel<CPLX, G32, MT, CAP>;
     else return zsolve_kernel<CPLX, G32, MT, CAP, true>;
 }
 }  // namespace
