@@ -82,8 +82,9 @@ struct PPMrPlan {
     unsigned magic[PP_MR_MAXPASS];  // division by the span of each pass
     int threads;
 };
-// the plan of a direction (half: its periodic half spectra); false where it has none
-bool pp_mr_plan(int n, int kind, bool half, PPMrPlan* p);
+// the plan of a direction (half: its periodic half spectra) of a grid of so many
+// points; false where it has none, or the generic kernel is faster
+bool pp_mr_plan(int n, int kind, bool half, long points, PPMrPlan* p);
 // data lines per CTA tile
 int pp_mr_lines(int n, int kind, const PPMrPlan& p);
 // one pass (a.tw and a.cs2 in its precision, strides and output strides set), in

@@ -29,14 +29,44 @@ const CtRange kCt[] = {
     {800, 1536, pp_launch_mr_ct_e_f64, pp_launch_mr_ct_e_f32},
 };
 
+// the lengths of pp_mr_ct_*.cu
+bool compiled(int n)
+{
+    static const short lengths[] = {40,  48,  50,  54,  60,  72,  80,  90,  96,  100, 108, 120, 144,  150,  160,  162,  180,
+                                    192, 200, 216, 240, 250, 270, 288, 300, 320, 324, 360, 384, 400,  432,  450,  480,  500,
+                                    540, 576, 600, 640, 720, 750, 768, 800, 864, 900, 960, 1000, 1152, 1200, 1280, 1536};
+    for (int c : lengths)
+        if (c == n) return true;
+    return false;
+}
+
+// Whether a plan is faster than the generic kernel (pp_linepass.cu).  Known at
+// compile time, or with a radix 11 or 13 (p^2 work a butterfly there): always.  Read at
+// run time, its passes are calls of their own at 128 registers, which a grid waits
+// for that fills the GPU only once or twice, and complex lines of three passes longer
+// than that.  Two passes of a direction, planned to generic:
+//   real, N x 64 x 8, x 24, x 80, x 256:  25 1.67, 1.59, 1.18, 0.81; 45 1.41, 1.40,
+//     0.94, 0.67; 105 1.02, 0.98, 0.65, 0.59; 315 1.38, 0.81, 0.99, 0.62; 42 (half
+//     length) 1.01, 1.02, 0.73, 0.51
+//   complex y, 64 x N x 8 .. 256:  45 1.37, 1.27, 1.19, 0.88; 315 1.33, 1.14, 1.38,
+//     1.28; 448 1.15, 1.00, 1.27, 1.12; x 800: 125 1.50, 135 0.82, 225 0.77, 189 1.03
+// Solves with the planned kernel always: 25^2 x 40 N-N 57 us and 37, 45^2 x 40 P-P 47
+// and 35, 315 x 64 x 40 P-P 105 and 80, 125 x 128 x 64 P-P 89 and 76.
+bool pays(int n, bool cplx, const PPMrPlan& p, long points)
+{
+    if (compiled(n) || n % 11 == 0 || n % 13 == 0) return true;
+    return points >= (cplx && p.npass > 2 ? 8000000L : 350000L);
+}
+
 }  // namespace
 
-bool pp_mr_plan(int n, int kind, bool half, PPMrPlan* p)
+bool pp_mr_plan(int n, int kind, bool half, long points, PPMrPlan* p)
 {
     *p = PPMrPlan{};
     const bool odd = n & 1;
     if ((half || pp_kind_is_quarter(kind)) && odd) return false;
     *p = pp_mr::make_plan((half || (kind != PP_KIND_FFT && !odd)) ? n / 2 : n);
+    if (p->m > 0 && !pays(n, kind == PP_KIND_FFT && !half, *p, points)) *p = PPMrPlan{};
     return p->m > 0;
 }
 

@@ -224,7 +224,7 @@ cudaError_t na_line_pass(PPLinePassArgs a, const NaDir& d, const double2* tw, co
         return pp_launch_line_pass_pow2<double, double, double>(a, inverse, strided, st);
     }
     PPMrPlan mr;
-    if ((d.kind == PP_KIND_FFT || !out_cplx || (inverse && !strided)) && pp_mr_plan(d.n, d.kind, false, &mr)) {
+    if ((d.kind == PP_KIND_FFT || !out_cplx || (inverse && !strided)) && pp_mr_plan(d.n, d.kind, false, (long)a.nx * a.ny * a.nz, &mr)) {
         a.tw = tw;
         a.cs2 = cs;
         return pp_mr_line_pass(a, mr, inverse, strided, in_cplx, out_cplx, false, st);

@@ -321,8 +321,9 @@ int build_dir(pp_solver_s* h, DirTables& t, int n, int kind)
         t.f2.tw = t.tw2.as<double2>();
     }
     if (t.n1 == 0) {
-        pp_mr_plan(n, kind, false, &t.mr);
-        if (kind == PP_KIND_FFT) pp_mr_plan(n, kind, true, &t.mrh);
+        const long points = (long)h->nx * h->ny * h->nz;
+        pp_mr_plan(n, kind, false, points, &t.mr);
+        if (kind == PP_KIND_FFT) pp_mr_plan(n, kind, true, points, &t.mrh);
     }
     t.fft.n = nf;
     t.fft.npass = (int)r.size();
