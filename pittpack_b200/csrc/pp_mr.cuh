@@ -448,9 +448,10 @@ PP_D void mr_body(const PPLinePassArgs& a, const PPMrPlan& pl)
     auto half_at = [&](int j) -> Real& { return rcol[2 * ((j >> 1) * LP) + (j & 1)]; };  // real j of the line
 
     // the forward x pass of the plain solve subtracts the Dirichlet lift (b = f dz^2 -
-    // lift, the dz^2 factor applied to the outputs)
+    // lift, the dz^2 factor applied to the outputs) from the few elements on a face:
+    // where they lie in the FFT input (1b), or as the odd lengths load them
     const PPLift& F = a.lift;
-    const bool face = !INV && !STR && a.rhs_scale && F.any &&
+    const bool face = K == K_PACK && !INV && !STR && sizeof(Real) == 8 && a.rhs_scale && F.any &&
                       (F.x0 || F.x1 || (F.z0 && plane == 0) || (F.z1 && plane == a.nz - 1) || (F.y0 && l0 == 0) ||
                        (F.y1 && l0 + nl >= a.ny));
     auto lift = [&](int d, int e) -> Real {
@@ -490,13 +491,7 @@ PP_D void mr_body(const PPLinePassArgs& a, const PPMrPlan& pl)
         for (int i = i0; i < M; i += G) col[i * LP] = mkc<C>(0, 0);
     } else if constexpr (K == K_CPLX) {
         auto st = [&](int i, C v) { col[i * LP] = v; };
-        if (a.in_cplx && !face) staged<U>(i0, M, G, [&](int i) { return srcc[i * es]; }, st);
-        else if (a.in_cplx)
-            staged<2>(i0, M, G, [&](int i) {
-                C v = srcc[i * es];
-                v.x -= lift(0, i);
-                return v;
-            }, st);
+        if (a.in_cplx) staged<U>(i0, M, G, [&](int i) { return srcc[i * es]; }, st);
         else staged<U>(i0, M, G, [&](int i) { return mkc<C>(X(i), (Real)0); }, st);
     } else if constexpr (!STR && (K == K_HALF || K == K_Q4 || K == K_REAL) && (K == K_Q4 || !INV)) {
         // contiguous reals, in pairs x_{2i}, x_{2i+1}
@@ -517,7 +512,7 @@ PP_D void mr_body(const PPLinePassArgs& a, const PPMrPlan& pl)
                 half_at(dst2 ? M - 1 - i : N - 1 - i) = v.y;
             }
         };
-        if (a.vec16 && !face) staged<U>(i0, M, G, [&](int i) { return reinterpret_cast<const C*>(src)[i]; }, st);
+        if (a.vec16) staged<U>(i0, M, G, [&](int i) { return reinterpret_cast<const C*>(src)[i]; }, st);
         else staged<2>(i0, M, G, [&](int i) { return mkc<C>(X(2 * i), X(2 * i + 1)); }, st);
     } else if constexpr (K == K_Q4) {
         staged<U>(i0, M, G, [&](int i) { return mkc<C>(X(2 * i), X(N - 1 - 2 * i)); },
@@ -622,6 +617,45 @@ PP_D void mr_body(const PPLinePassArgs& a, const PPMrPlan& pl)
                 const int ec = dst2 ? N - 1 - M + k : M - k, ed = dst2 ? N - 1 - M - k : M + k;
                 return Quad<Real, C>{X(ea), X(eb), X(ec), X(ed < 0 ? 0 : ed), __ldg(&cs[k]), __ldg(&tw[k])};
             }, use);
+        }
+    }
+    // ---- 1b. the lift, where the face's elements lie: tests between the loads or in
+    //      their use cost every grid with boundary data on x (320^3 D-D, forward x
+    //      0.298 ms, 0.152 now, 0.112 without data) and registers every other one ----------
+    if constexpr (!INV && !STR && K != K_PACK && sizeof(Real) == 8) {
+        if (a.rhs_scale && F.any &&
+            (F.x0 || F.x1 || (F.z0 && plane == 0) || (F.z1 && plane == a.nz - 1) || (F.y0 && l0 == 0) ||
+             (F.y1 && l0 + nl >= a.ny))) {
+            __syncthreads();
+            const int j = l0 + l;  // y row of the line
+            const double* zr = (F.z0 && plane == 0) ? F.z0 + (long)a.nx * j
+                               : (F.z1 && plane == a.nz - 1) ? F.z1 + (long)a.nx * j : nullptr;
+            const double* yr = (F.y0 && j == 0) ? F.y0 + (long)a.nx * plane
+                               : (F.y1 && j == a.ny - 1) ? F.y1 + (long)a.nx * plane : nullptr;
+            auto take = [&](int e) {
+                double s = zr ? zr[e] : 0.0;
+                if (F.x0 && e == 0) s += F.x0[j + (long)a.ny * plane];
+                if (F.x1 && e == N - 1) s += F.x1[j + (long)a.ny * plane];
+                if (yr) s += yr[e];
+                const double v = s / (a.dz * a.dz);
+                const int i = e >> 1;
+                if constexpr (K == K_CPLX) {
+                    rcol[2 * e * LP] -= v;
+                } else if constexpr (K == K_HALF) {
+                    half_at(e) -= v;
+                } else if constexpr (K == K_Q4) {
+                    rcol[(e & 1) ? 2 * ((M - 1 - i) * LP) + (rev ? 0 : 1) : 2 * (i * LP) + (rev ? 1 : 0)] -= v;
+                } else {
+                    Real& x = half_at((e & 1) ? (dst2 ? M - 1 - i : N - 1 - i) : dst2 ? M + i : i);
+                    x = dst2 && !(e & 1) ? x + v : x - v;
+                }
+            };
+            if (live && (zr || yr)) {
+                for (int e = i0; e < N; e += G) take(e);
+            } else if (live && i0 == 0) {
+                if (F.x0) take(0);
+                if (F.x1) take(N - 1);
+            }
         }
     }
     __syncthreads();
@@ -820,9 +854,12 @@ __global__ void __launch_bounds__(256, 2) mr_kernel(PPLinePassArgs a, PPMrPlan p
     mr_body<Real, K, INV, STR, 0>(a, p);
 }
 // planned at compile time: M points
-constexpr int ct_blocks(int points, int threads) { return (points <= 10 ? 768 : points <= 12 ? 640 : 512) / threads; }
+constexpr int ct_blocks(int points, int threads, bool f32_forward)
+{
+    return (points <= 10 ? 768 : points <= 12 || f32_forward ? 640 : 512) / threads;
+}
 template <typename Real, int K, bool INV, bool STR, int M>
-__global__ void __launch_bounds__(Plan<M>::P.threads, ct_blocks(Plan<M>::points(), Plan<M>::P.threads))
+__global__ void __launch_bounds__(Plan<M>::P.threads, ct_blocks(Plan<M>::points(), Plan<M>::P.threads, sizeof(Real) == 4 && !INV && !STR))
 mrc_kernel(PPLinePassArgs a)
 {
     mr_body<Real, K, INV, STR, M>(a, PPMrPlan{});
