@@ -54,7 +54,7 @@ void batch_free(pp_batch_s* b)
     delete b;
 }
 
-// How many grids run at once, at most 'branches': as many as keep their spectra
+// How many grids run at once, at most 'branches': of plain solves as many as keep their spectra
 // in three quarters of L2 together (right-hand sides and solutions pass through
 // the rest).  A grid's passes hand the two spectra from one to the next through
 // L2; past its capacity every pass goes to memory and back (48 grids of 32 ..
@@ -64,8 +64,14 @@ void batch_free(pp_batch_s* b)
 // and 1.93, 8 of 256^3 2.20 and 2.49, 6 of 256 x 256 x 320 2.07 and 2.21, 16 mixed
 // of 128 .. 320 3.42 and 3.72; with workspaces of their own 2, 3, 4 and 8 branches
 // of these were within 6 %).
+// Refined solves run as many as asked for: a sweep's residual, sums and zero-mode
+// column are small launches that wait for one another, and more grids fill them
+// (ms at 3, 6, 8 and 16 branches: 48 uneven grids 4.09, 3.19, 3.19 and 3.56, 96 of
+// them 9.15, 7.48, 7.59 and 8.84, 24 of 128^3 2.25, 1.84, 1.84 and 1.84, 64 of 64^3
+// 3.20, 1.83, 1.46 and 0.95, 8 of 256^3 4.64, 4.62, 4.59 and 4.59).
 int branches_in_l2(const pp_batch_item* items, int n, bool refined, int branches)
 {
+    if (refined) return branches;
     int dev = 0, l2 = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess ||
         l2 <= 0)
@@ -73,10 +79,10 @@ int branches_in_l2(const pp_batch_item* items, int n, bool refined, int branches
     double bytes = 0.0;
     for (int i = 0; i < n; ++i) {
         // two real spectra (half spectra of a periodic x as much), the second one
-        // complex for a periodic y alone; refined: FP32 spectra and residual, u
+        // complex for a periodic y alone
         if (items[i].nx <= 0 || items[i].ny <= 0 || items[i].nz <= 0) continue;  // rejected later
         const bool wide = items[i].bc[2] == 'P' && items[i].bc[0] != 'P';
-        bytes += (refined ? 20.0 : wide ? 24.0 : 16.0) * items[i].nx * (double)items[i].ny * items[i].nz;
+        bytes += (wide ? 24.0 : 16.0) * items[i].nx * (double)items[i].ny * items[i].nz;
     }
     const double fit = bytes > 0 ? 0.75 * l2 * n / bytes : branches;
     return fit >= branches ? branches : std::min(branches, std::max(2, (int)fit));
