@@ -41,20 +41,24 @@ bool compiled(int n)
 }
 
 // Whether a plan is faster than the generic kernel (pp_linepass.cu).  Known at
-// compile time, or with a radix 11 or 13 (p^2 work a butterfly there): always.  Read at
+// compile time, or with a radix 11 or 13 (p^2 work a butterfly there): always; also
+// even DCT-II / DST-II lengths, whose passes are level on the smallest grids and whose
+// z solve gains the z-tiled spectrum (50 x 42 x 37 36.9 and 35.3 us).  Read at
 // run time, its passes are calls of their own at 128 registers, which a grid waits
 // for that fills the GPU only once or twice, and complex lines of three passes longer
 // than that.  Two passes of a direction, planned to generic:
 //   real, N x 64 x 8, x 24, x 80, x 256:  25 1.67, 1.59, 1.18, 0.81; 45 1.41, 1.40,
-//     0.94, 0.67; 105 1.02, 0.98, 0.65, 0.59; 315 1.38, 0.81, 0.99, 0.62; 42 (half
-//     length) 1.01, 1.02, 0.73, 0.51
+//     0.94, 0.67; 105 1.02, 0.98, 0.65, 0.59; 315 1.38, 0.81, 0.99, 0.62; even 42 1.01,
+//     1.02, 0.73, 0.51, its DCT-IV 1.13, 1.17, 0.86, 0.62
 //   complex y, 64 x N x 8 .. 256:  45 1.37, 1.27, 1.19, 0.88; 315 1.33, 1.14, 1.38,
 //     1.28; 448 1.15, 1.00, 1.27, 1.12; x 800: 125 1.50, 135 0.82, 225 0.77, 189 1.03
 // Solves with the planned kernel always: 25^2 x 40 N-N 57 us and 37, 45^2 x 40 P-P 47
 // and 35, 315 x 64 x 40 P-P 105 and 80, 125 x 128 x 64 P-P 89 and 76.
-bool pays(int n, bool cplx, const PPMrPlan& p, long points)
+bool pays(int n, int kind, bool half, const PPMrPlan& p, long points)
 {
     if (compiled(n) || n % 11 == 0 || n % 13 == 0) return true;
+    if (n % 2 == 0 && (kind == PP_KIND_DCT2 || kind == PP_KIND_DST2)) return true;
+    const bool cplx = kind == PP_KIND_FFT && !half;
     return points >= (cplx && p.npass > 2 ? 8000000L : 350000L);
 }
 
@@ -66,7 +70,7 @@ bool pp_mr_plan(int n, int kind, bool half, long points, PPMrPlan* p)
     const bool odd = n & 1;
     if ((half || pp_kind_is_quarter(kind)) && odd) return false;
     *p = pp_mr::make_plan((half || (kind != PP_KIND_FFT && !odd)) ? n / 2 : n);
-    if (p->m > 0 && !pays(n, kind == PP_KIND_FFT && !half, *p, points)) *p = PPMrPlan{};
+    if (p->m > 0 && !pays(n, kind, half, *p, points)) *p = PPMrPlan{};
     return p->m > 0;
 }
 

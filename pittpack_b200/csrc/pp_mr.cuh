@@ -26,7 +26,8 @@
 // 200, 300, 500, 1000, the multiples 48, 96, 144, 192, 288, 384, 576, 768 and
 // their like, even and of factors 2, 3 and 5) are instances with the plan known at
 // compile time; the others take one kernel that reads it at run time, its passes
-// functions of their own.
+// functions of their own, where that beats the generic kernel (pays, pp_mr.cu).  Long
+// contiguous lines m 2^k run the register kernel instead (pp_lpm_takes).
 //
 // What bounds it is the shared-memory pipe (about 8 + 8 + 16 passes + 8 + 8 bytes
 // a point, 50 - 68 % busy), then the latency of the phases at 14 to 20 warps

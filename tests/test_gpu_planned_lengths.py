@@ -1,6 +1,8 @@
 """The transform pass planned from the length (pp_mr.cuh): lengths planned at
-compile time and at run time, even (half-length FFT) and odd (two lines per
-FFT), every radix, in x and in y, with partial tiles, buffers off the widest
+compile time and at run time (on grids this small the even DCT / DST ones and those
+with a factor 11 or 13; the others take the generic kernel here, and the plan in
+test_gpu_planned_runtime.py),
+even (half-length FFT) and odd (two lines per FFT), every radix, in x and in y, with partial tiles, buffers off the widest
 accesses, padded spectrum columns and complex right-hand sides, against the
 oracle: relative L2 <= 1e-12 in FP64, <= 1e-10 for the refined solve."""
 import numpy as np
