@@ -70,7 +70,7 @@ def _run(target, world, *args):
 
 CASES = [(2, 16, 12, 10, "NNNNDD", (0, 1, 0, 1, 0, 1)),        # Dirichlet z: each end face on one slab
          (2, 32, 20, 9, "PPPPDD", (0, 1, 0, 2, -1, 1)),        # half spectra, complex y / z, uneven slabs
-         (2, 12, 10, 8, "DDNNPP", (0, 1, 0, 1, 0, 1)),         # periodic z (Sherman-Morrison on whole columns)
+         (2, 12, 10, 8, "DDNNPP", (0, 1, 0, 1, 0, 1)),         # periodic z (the ring of lanes on whole columns)
          (3, 24, 18, 15, "NDDNNN", (0, 2, 0, 1, 0, 1)),        # three ranks, quarter-wave x
          (3, 20, 10, 12, "NNNNNN", (0, 1, 0, 1, 0, 1))]        # the singular zero-mode column on one rank
 
