@@ -35,12 +35,13 @@
 // loads and uses in turn 200^3 took 0.297 ms, at run time 0.42).  FP64, ms per
 // solve, before (pp_linepass.cu; * a register kernel for m 2^k) -> run-time plan
 // -> compile-time plan:
-//   200^3 N-N            0.888 -> 0.34 -> 0.189    384^3 N-N *  1.25 -> 1.08
-//   500 x 400 x 300 D-D  6.48      ->     1.34     192^3 P-P *  0.184 -> 0.152
-//   1000 x 800 x 100     9.06  -> 4.2  -> 1.78     960^2 x 128 * 5.05 -> 3.52
+//   200^3 N-N            0.888 -> 0.34 -> 0.188    384^3 N-N *  1.25 -> 1.08
+//   500 x 400 x 300 D-D  6.48      ->     1.33     192^3 P-P *  0.184 -> 0.146
+//   1000 x 800 x 100     9.06  -> 4.2  -> 1.78     960^2 x 128 * 5.05 -> 3.02 (x by the
+//                                                  register kernel; 3.52 all planned)
 // The generic kernel of before (one complex FFT of N per real line, radix <= 8 in
 // two ping-pong buffers, half a dozen passes over them) stays for larger prime
-// factors and for odd lengths of DCT-IV / DST-IV.
+// factors, for odd lengths of DCT-IV / DST-IV and for small grids (pays).
 #pragma once
 
 #include "pp_rhalf.cuh"
